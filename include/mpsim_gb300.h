@@ -83,8 +83,8 @@ typedef struct {
                               MPS_PRECISION_MIXED                          */
     int32_t lq_off;        /* nonzero: no LQ preconditioning (the sweeps run
                               on theta itself)                              */
-    int32_t block_request; /* Jacobi block width of the plain form for slots
-                              of 512 / 576 rows: 0 (default) = 16, or 8     */
+    int32_t block_request; /* 0, 8 or 16; the plain form's sweeps use 8-column
+                              blocks for each                              */
 } mps_svd_params;
 
 /* mps_svd_params.precision.

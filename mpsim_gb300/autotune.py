@@ -5,9 +5,9 @@ The choices it makes per call (fields of ``mps_svd_params``):
 * ``lq_off``        -- run the Jacobi sweeps on theta itself instead of its L
   factor (the LQ factorisation costs panels on a few SMs; the sweeps it saves
   depend on the shape);
-* ``block_request`` -- 16- or 8-column blocks in the plain sweep kernel for
-  512 / 576-row slots (fewer registers and more resident CTAs against more
-  rounds per sweep);
+* ``block_request`` -- the plain sweeps' block width for 512 / 576-row slots; the
+  library takes 0, 8 and 16 and uses 8-column blocks for each, so today its
+  candidates measure alike;
 * ``precision``     -- for ``MPS(precision="auto")``: the plain FP32 sweeps or
   the tensor-core block sweeps, whichever is faster for that shape and batch.
 

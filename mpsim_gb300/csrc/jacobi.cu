@@ -11,7 +11,9 @@
 // (circle-method round robin), so every pair of columns is rotated exactly
 // once per sweep.  One persistent launch runs a whole sweep: CTAs take
 // (round, job, block pair) items in round-major order and wait (bounded) for
-// the two blocks' previous round.
+// the two blocks' previous round.  Slots of up to kGramRows rows take the sweep
+// kernel of gramsweep.cu, whose visits work on the pair's Gram matrix; the one
+// here serves longer columns, whose visits do not fit beside it.  In it
 //  * round 0 ("full" visit): the CTA stages its 2*BC columns in shared memory
 //    and rotates all pairs among them -- the intra-block pairs of every block
 //    (round 0's pairs cover each block once) and the first inter-block pairs;
@@ -764,14 +766,18 @@ presort_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int npow2, int b
     }
     if (g.vstamp) {
         // a block whose set of columns changes counts as changed (its pairs
-        // are not the ones last checked); moves inside a block do not
+        // are not the ones last checked); moves inside a block do not, except
+        // for the Gram sweeps, whose block products go by position
         int* oldpos = reinterpret_cast<int*>(key);     // the keys are no longer needed
         for (int i = tid; i < C; i += PRESORT_T) oldpos[__ldcg(g.cmap + (size_t)j * g.cslot + i)] = i;
         __syncthreads();
         int* vst = g.vstamp + (size_t)j * g.nbmax;
+        int2* bst = g.gstate + (size_t)j * g.nbmax;
         for (int c = tid; c < C; c += PRESORT_T) {
             const int ob = oldpos[idx[c]] / bc, nb = c / bc;
-            if (ob != nb) {
+            if (g.gstate) {
+                if (oldpos[idx[c]] != c) bst[ob].y = bst[nb].y = tpre;
+            } else if (ob != nb) {
                 vst[ob] = tpre;
                 vst[nb] = tpre;
             }
@@ -1346,23 +1352,6 @@ int launch_sweep(const mps_2q_job* jobs, int njobs, int rounds, int pairs, const
     return MPS_OK;
 }
 
-typedef int (*sweep_fn)(const mps_2q_job*, int, int, int, const TwoQGeom&, float, int,
-                        const SweepSync&, int, cudaStream_t);
-
-sweep_fn pick_sweep(int lw, int block_request) {
-    if (block_request == 8 && lw > 256 && lw <= 576)
-        return lw <= 512 ? launch_sweep<8, 16> : launch_sweep<8, 18>;
-    if (lw <= 576) {
-        if (lw <= 64) return launch_sweep<16, 2>;
-        if (lw <= 128) return launch_sweep<16, 4>;
-        if (lw <= 256) return launch_sweep<16, 8>;
-        if (lw <= 512) return launch_sweep<16, 16>;
-        return launch_sweep<16, 18>;
-    }
-    if (lw <= 1024) return launch_sweep<8, 32>;
-    return launch_sweep<8, 56>;
-}
-
 typedef int (*visit_fn)(const mps_2q_job*, int, int, const TwoQGeom&, int, float, int, cudaStream_t);
 
 // Block width and register rows for a working column length lw (<= 1792).
@@ -1383,7 +1372,7 @@ visit_fn pick_visit(int lw, int* bc) {
 struct Layout {
     int lslot, cslot;
     size_t off_X, off_V, off_T, off_sig, off_perm, off_cmap, off_cnrm, off_off, off_done, off_need,
-        off_counter, off_scale, off_nrm2, off_sync, off_vst, off_qst, off_P, total;
+        off_counter, off_scale, off_nrm2, off_sync, off_vst, off_gst, off_qst, off_gblk, off_gact, off_P, total;
     int nbmax, qstride;
 };
 
@@ -1396,7 +1385,7 @@ int slot_rows(int L) {
     return (int)align_up((size_t)L, 32);
 }
 
-Layout make_layout(int njobs, int max_m, int max_n, bool pieces = false) {
+Layout make_layout(int njobs, int max_m, int max_n, bool pieces = false, bool gram = true) {
     Layout lo;
     const int L = max(max_m, max_n), C = min(max_m, max_n);
     lo.lslot = slot_rows(max(L, 1));
@@ -1423,7 +1412,14 @@ Layout make_layout(int njobs, int max_m, int max_n, bool pieces = false) {
     // visit skipping: a stamp per column block and per (round, pair)
     lo.qstride = lo.nbmax * (lo.nbmax / 2);
     lo.off_vst = o; o = align_up(o + nj * lo.nbmax * sizeof(int), 256);
+    lo.off_gst = o;
+    if (gram && lo.lslot <= kGramRows) o = align_up(o + nj * lo.nbmax * sizeof(int2), 256);
     lo.off_qst = o; o = align_up(o + nj * lo.qstride * sizeof(int), 256);
+    // the Gram sweeps' products within the column blocks
+    lo.off_gblk = o;
+    if (gram && lo.lslot <= kGramRows) o = align_up(o + nj * kGramBlock * lo.cslot * sizeof(cf), 256);
+    lo.off_gact = o;
+    if (gram && lo.lslot <= kGramRows) o = align_up(o + (nj + 1) * sizeof(int4), 256);
     // the mixed form's bf16 piece planes of X (3 per job)
     lo.off_P = o;
     if (pieces) o = align_up(o + nj * 3 * 2 * (size_t)lo.lslot * lo.cslot * sizeof(uint16_t), 256);
@@ -1499,6 +1495,11 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
     g.qstamp = reinterpret_cast<int*>(ws + lo.off_qst);
     g.nbmax = lo.nbmax;
     g.qstride = lo.qstride;
+    const int block_request = params ? params->block_request : 0;
+    const bool gram = lo.lslot <= kGramRows;
+    g.gblk = gram ? reinterpret_cast<cf*>(ws + lo.off_gblk) : nullptr;
+    g.gstate = gram ? reinterpret_cast<int2*>(ws + lo.off_gst) : nullptr;
+    g.gact = gram ? reinterpret_cast<int4*>(ws + lo.off_gact) : nullptr;
     g.P = mixed_req ? reinterpret_cast<uint16_t*>(ws + lo.off_P) : nullptr;
     g.pplane = (size_t)2 * lo.lslot * lo.cslot;
 
@@ -1520,13 +1521,10 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
     if (params && params->precision != MPS_PRECISION_PLAIN && !mixed)
         return fail(MPS_ERR_ARG, "mps_apply_2q_batch: unknown precision");
     const int lw = lo.lslot;
-    int bc = 16;
-    (void)pick_visit(lw, &bc);
-    const int block_request = params ? params->block_request : 0;
     if (block_request != 0 && block_request != 8 && block_request != 16)
         return fail(MPS_ERR_ARG, "mps_apply_2q_batch: block_request must be 0, 8 or 16");
-    sweep_fn sweep = pick_sweep(lw, block_request);
-    if (block_request == 8 && lw > 256 && lw <= 576) bc = 8;
+    constexpr int bc = 8;
+    static_assert(kGramBlock == bc, "one block width for both sweep kernels");
     // MPS_PRECISION_MIXED: the left-canonical tall jobs of 64+ columns take
     // the tensor-core sweeps (32-column blocks), the others the SIMT ones, in
     // the same sweep loop
@@ -1594,21 +1592,27 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
         // (unknown, so both run, before the first read and under capture)
         bool tc_left = true, simt_left = true;
         for (sweeps = 1; sweeps <= max_sweeps; ++sweeps) {
-            MPS_CUDA_CHECK(cudaMemsetAsync(g.counter, 0, sizeof(int), s));
-            if (mixed) MPS_CUDA_CHECK(cudaMemsetAsync(g.counter + 4, 0, 2 * sizeof(int), s));
             if (cmax > 2 * bc) {
                 presort_kernel<<<njobs, PRESORT_T, sort_smem, s>>>(jobs, g, npow2, bc,
                                                                    sweeps * tbase_stride);
                 MPS_LAUNCH_CHECK("presort_kernel");
             }
-            MPS_CUDA_CHECK(cudaMemsetAsync(sync.block_round, 0xff,
-                                           (size_t)njobs * lo.nbmax * sizeof(int), s));
+            if (gram) {
+                if (int e = gram_begin_launch(jobs, njobs, g, sync, s)) return e;
+            } else {
+                MPS_CUDA_CHECK(cudaMemsetAsync(g.counter, 0, sizeof(int), s));
+                if (mixed) MPS_CUDA_CHECK(cudaMemsetAsync(g.counter + 4, 0, 2 * sizeof(int), s));
+                MPS_CUDA_CHECK(cudaMemsetAsync(sync.next_item, 0, (mixed ? 1 : 2) * sizeof(int), s));
+            }
+            if (mixed || !gram)
+                MPS_CUDA_CHECK(cudaMemsetAsync(sync.block_round, 0xff,
+                                               (size_t)njobs * lo.nbmax * sizeof(int), s));
             if (mixed) {
                 // the tensor-core jobs: one persistent launch per sweep with
-                // the same round flags and visit stamps as the SIMT form (its
-                // own item counter, counter[2]); X is split into its bf16
-                // pieces before the first sweep.  An expired wait stays in
-                // sync.error until the call returns.
+                // round flags and visit stamps of its own (its own item
+                // counter, counter[2]); X is split into its bf16 pieces before
+                // the first sweep.  An expired wait stays in sync.error until
+                // the call returns.
                 if (sweeps == 1) {
                     MPS_CUDA_CHECK(cudaMemsetAsync(sync.error, 0, sizeof(int), s));
                     if (int e = tc_split_launch(jobs, njobs, g, s)) return e;
@@ -1621,14 +1625,14 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
                                          sweeps * tbase_stride, s);
                     if (rc) return rc;
                 }
-                MPS_CUDA_CHECK(cudaMemsetAsync(sync.next_item, 0, sizeof(int), s));
-            } else {
-                MPS_CUDA_CHECK(cudaMemsetAsync(sync.next_item, 0, 2 * sizeof(int), s));
             }
             // the SIMT jobs (all of them in the plain form): one persistent
             // launch runs every round of the sweep
             if (simt_left) {
-                rc = sweep(jobs, njobs, rounds, pairs, g, tol2, lw, sync, sweeps * tbase_stride, s);
+                rc = gram ? gram_sweep_launch(njobs, rounds, pairs, g, tol2, sync,
+                                              sweeps * tbase_stride, s)
+                          : launch_sweep<8, 56>(jobs, njobs, rounds, pairs, g, tol2, lw, sync,
+                                                sweeps * tbase_stride, s);
                 if (rc) return rc;
             }
             sweep_end_kernel<<<(njobs + 255) / 256, 256, 0, s>>>(jobs, g, njobs, tol2, sync.error);
@@ -1771,7 +1775,7 @@ extern "C" int mps_apply_2q_batch_noalloc(void* stream, const mps_2q_job* jobs, 
     if (d < 1 || d > 64) return fail(MPS_ERR_ARG, "mps_apply_2q_batch_noalloc: qudit dimension must be 1..64");
     if (max_m <= 0 || max_n <= 0)
         return fail(MPS_ERR_ARG, "mps_apply_2q_batch_noalloc: max_m/max_n must be positive");
-    const Layout lo = make_layout(njobs, max_m, max_n, false);
+    const Layout lo = make_layout(njobs, max_m, max_n, false, false);
     if (lo.lslot > 1792)
         return fail(MPS_ERR_ARG, "mps_apply_2q_batch_noalloc: merged matrix longer than 1792 rows "
                                  "is beyond this build's shared-memory Jacobi kernel");
@@ -1808,6 +1812,9 @@ extern "C" int mps_apply_2q_batch_noalloc(void* stream, const mps_2q_job* jobs, 
     g.qstamp = nullptr;
     g.nbmax = lo.nbmax;
     g.qstride = lo.qstride;
+    g.gblk = nullptr;
+    g.gstate = nullptr;
+    g.gact = nullptr;
     g.P = nullptr;
     g.pplane = 0;
     g.tc_mode = 0;

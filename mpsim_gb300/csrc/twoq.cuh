@@ -41,6 +41,17 @@ struct TwoQGeom {
     int* vstamp;      // njobs * nbmax: last time a column block changed
     int* qstamp;      // njobs * qstride: last time visit (round, pair) rotated nothing
     int nbmax, qstride;
+    // Products within each 8-column block (block b of job j: 8 x 8 complex at
+    // gblk + (j * cslot / 8 + b) * 64, the entries above the diagonal), kept by
+    // the Gram sweep kernel beside the columns; null where unused
+    cf* gblk;
+    // njobs * nbmax, the Gram sweeps' progress (null where unused): x, the last
+    // time (as above) a visit of the block ended; y, the last time it changed
+    int2* gstate;
+    // The jobs the Gram sweeps have left, compacted before every sweep: entry 0
+    // is (count, rounds, pairs, 0) over them, entry 1 + i job i's (index, L, C,
+    // rows of V); njobs + 1 entries, null where unused
+    int4* gact;
     // MPS_PRECISION_MIXED only (null otherwise): X split into three bf16
     // piece planes per job, plane i of job j at P + (3 j + i) * pplane, each
     // laid out like X (column c = 2 lslot bf16 at c * 2 lslot); during the
@@ -90,6 +101,19 @@ constexpr float kZeroSigma = 1e-30f;
 // from the final columns (lq.cu); the sweeps then need fewer passes.
 int lq_precondition(const mps_2q_job* jobs, int njobs, int max_m, int max_n, const TwoQGeom& g,
                     cudaStream_t s);
+
+// One sweep of the SIMT jobs by Gram visits (gramsweep.cu): slots of up to
+// kGramRows rows, blocks of kGramBlock columns; arguments as for jacobi.cu's
+// sweep kernel.
+constexpr int kGramRows = 1024;
+constexpr int kGramBlock = 8;
+// gram_begin_launch, before each sweep, lists the jobs left in g.gact and clears
+// counter[0] (and [4], [5] of a mixed call), the item counter and, in the plain
+// form, the error word.
+int gram_begin_launch(const mps_2q_job* jobs, int njobs, const TwoQGeom& g, const SweepSync& sync,
+                      cudaStream_t s);
+int gram_sweep_launch(int njobs, int rounds, int pairs, const TwoQGeom& g,
+                      float tol2, const SweepSync& sync, int tbase, cudaStream_t s);
 
 // Tensor-core block sweeps (tcjacobi.cu): one persistent launch runs every
 // round of one sweep of the tc_job() jobs, 32-column blocks, with the sweep

@@ -1,0 +1,42 @@
+"""Gram sweeps at the sizes where their tiles end: 8-column blocks (padding
+blocks, odd block counts), 64-row tasks of the apply warps, the slot lengths, and
+jobs that accumulate V.  Checked like test_gpu_svd_kernel.py's jobs (same
+tolerances) against complex128 LAPACK.
+"""
+import numpy as np
+import pytest
+
+from mpsim_gb300 import _native
+from test_gpu_svd_kernel import check_job, make_job_inputs, run_batch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("chil,chir", [
+    (1, 2), (4, 4), (4, 5), (8, 9), (12, 12), (16, 17), (31, 32), (32, 33), (36, 37), (63, 65),
+    (64, 64), (65, 60), (128, 100), (129, 128), (250, 140), (257, 255), (300, 40)])
+@pytest.mark.parametrize("lc", [True, False])
+def test_sizes(built_lib, cuda, chil, chir, lc):
+    """theta of 2 chil x 2 chir, from 2 x 4 to 600 x 80, in both forms."""
+    rng = np.random.default_rng(1000 * chil + chir)
+    chim = max(chil, chir)
+    a, b, g = make_job_inputs(rng, chil, chim, chir, 2, scale=1.0 / chim)
+    k = max(1, min(chil, chir))
+    rc, res, _ = run_batch(built_lib, cuda, [(a, b, g, k, lc)])
+    assert rc == 0, _native.last_error()
+    check_job((a, b, g, k, lc), res[0], 2)
+
+
+def test_mixed_shapes_in_one_call(built_lib, cuda):
+    """Jobs of different lengths, widths and forms in one slot class, more visits
+    than the SMs have slots."""
+    rng = np.random.default_rng(5)
+    specs = []
+    for q in range(70):
+        chil, chir = int(rng.integers(20, 65)), int(rng.integers(3, 65))
+        a, b, g = make_job_inputs(rng, chil, 64, chir, 2, scale=0.1)
+        specs.append((a, b, g, min(chil, chir), bool(q % 3)))
+    rc, res, _ = run_batch(built_lib, cuda, specs)
+    assert rc == 0, _native.last_error()
+    for spec, out in zip(specs, res):
+        check_job(spec, out, 2)
