@@ -199,7 +199,11 @@ int mps_wavefunction(void* stream, const mps_c64* const* sites,
 
 /* Amplitudes <x|psi> for nbits bitstrings (bits_dev: nbits x n int8,
  * row-major) into out_dev (nbits complex64).  workspace:
- * 2 * nbits * d * max_chi complex64. */
+ * 2 * nbits * d * max_chi complex64, or better
+ * mps_amplitudes_workspace_bytes(), which leaves room to group the bitstrings
+ * by digit at every site (each then multiplies one of the site's d matrices
+ * instead of all). */
+size_t mps_amplitudes_workspace_bytes(int nbits, int max_chi, int n, int d);
 int mps_amplitudes(void* stream, const mps_c64* const* sites, const int* chis,
                    int n, int d, const int8_t* bits_dev, int nbits,
                    mps_c64* out_dev, void* workspace, size_t workspace_bytes);
@@ -248,8 +252,8 @@ int mps_tc_error(int* flag_out);
  * CTAs.  Blocks. */
 int mps_tc_profile(unsigned long long* out10, int reset);
 
-/* Workspace for mps_site_marginals: every left environment plus two
- * right environments and two (chi, d, chi) scratch tensors. */
+/* Workspace for mps_site_marginals: two environments a direction and, for
+ * each direction, a (chi_l, d, chi_r) product of every site. */
 size_t mps_marginals_workspace_bytes(const int* chis, int n, int d);
 
 /* The diagonal of every single-site reduced density matrix,

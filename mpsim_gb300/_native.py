@@ -76,6 +76,7 @@ SIGNATURES = {
     "mps_inner_product": (_I, [_P, _P, _P, _P, _P, _I, _I, _P, _SZ, _P]),
     "mps_wavefunction": (_I, [_P, _P, _P, _I, _I, _P, _P, _SZ]),
     "mps_amplitudes": (_I, [_P, _P, _P, _I, _I, _P, _I, _P, _P, _SZ]),
+    "mps_amplitudes_workspace_bytes": (_SZ, [_I, _I, _I, _I]),
     "mps_scale": (_I, [_P, _P, _SZ, ctypes.c_float, ctypes.c_float, _I]),
     "mps_cgemm": (_I, [_P, _I, _I, _I, _P, _LL, _LL, _I, _P, _LL, _LL, _I, _P, _LL, _LL, _I,
                        _LL, _LL, _LL]),

@@ -612,7 +612,8 @@ class MPS:
         chis = self._chis()
         mx = max(chis)
         d = self._qudit_dimension
-        ws = _WS.get(self._device, (nb * d * mx + 2 * nb * mx) * 8, "amp")
+        ws = _WS.get(self._device, self._lib().mps_amplitudes_workspace_bytes(
+            nb, mx, self._nqudits, d), "amp")
         bdev = torch.from_numpy(bits).to(self._device)
         out = torch.empty(nb, dtype=torch.complex64, device=self._device)
         _native.check(self._lib().mps_amplitudes(

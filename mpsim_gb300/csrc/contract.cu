@@ -9,8 +9,11 @@
 //   renormalize / dagger   mpsim/core.py:567-594, 502-505
 //   marginals for sample   mpsim/core.py:655-667 (reduced_density_matrix(i)
 //                          diagonal, core.py:596-653)
+#include <limits.h>
+
 #include <atomic>
 #include <string>
+#include <vector>
 
 #include "common.cuh"
 
@@ -170,9 +173,22 @@ __global__ void scale_kernel(cf* __restrict__ x, size_t count, cf alpha, int con
 // ---------------------------------------------------------------------------
 // Generic complex GEMM C = op(A) op(B) with arbitrary element strides and
 // optional conjugation, batched over blockIdx.z with element strides bsa,
-// bsb, bsc between batches (zero: the same matrix for every batch).  64x64
-// tile, K chunks of 16, 256 threads, each thread 4x4 outputs at
-// (ty + 16i, tx + 16j).
+// bsb, bsc between batches (zero: the same matrix for every batch), or two
+// different products in one launch (the two directions of a sweep).
+//
+// 256 threads form TM x TN outputs, 4 x 4 a thread (rows ty + TM/4 i, columns
+// tx + TN/4 j), from K chunks copied into shared memory three ahead; KS groups of threads each take a share of every chunk and are summed at
+// the end, so that a 32 x 32 tile keeps all eight warps busy.
+//
+// What bounds it: the FP32 pipes for large products (64 x 64 tiles: 8 wavefronts
+// of shared-memory reads for 64 FMAs a thread), and the few tiles of the sweeps'
+// 256 x 512 x 256 steps otherwise -- there 32 x 32 tiles, and both directions
+// of a sweep in one launch, put work on every SM.  Measured (GB300) against one
+// direction at a time, 64 x 64 tiles and loads that were waited for chunk by
+// chunk: norm and overlap of a 64-site chi=256 state 14.3 -> 2.65 ms (FMA pipe
+// 53% busy, 74% of issue slots), marginals of 48 sites of chi=128 8.1 -> 0.96 ms
+// (the third product a site is gone too), 4096 amplitudes at chi=256 7.6 -> 3.1 ms
+// (half of the products were of digits not asked for).
 struct GemmArgs {
     int M, N, K;
     const cf* A;
@@ -187,80 +203,279 @@ struct GemmArgs {
     long long bsa, bsb, bsc;
 };
 
-__global__ void __launch_bounds__(256) cgemm_kernel(GemmArgs g) {
-    __shared__ cf As[16][64];
-    __shared__ cf Bs[16][64];
-    g.A += blockIdx.z * g.bsa;
-    g.B += blockIdx.z * g.bsb;
-    g.C += blockIdx.z * g.bsc;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
+// GATHER (sampled amplitudes): row i of A and C is row rows[i] of the arrays
+// (negative: none), and B is shifted by digit * bdig, one digit per TM rows
+// (negative: no row; >= ndig: the product is zero).
+struct GemmGather {
+    const int* rows;
+    const int* digit;
+    long long bdig;
+    int ndig;
+};
+
+__device__ __forceinline__ void copy8_async(uint32_t dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+                 : "memory");
+}
+
+struct GemmLaunch {
+    GemmArgs p[2];
+    int two;                    // blockIdx.z selects p[0] or p[1], else the batch
+    GemmGather ga;
+};
+
+// acc += a b, or a conj(b).
+template <bool CONJ>
+__device__ __forceinline__ void cfma_op(cf& acc, cf a, cf b) {
+    if (CONJ) {
+        acc.x = fmaf(a.x, b.x, fmaf(a.y, b.y, acc.x));
+        acc.y = fmaf(a.y, b.x, fmaf(-a.x, b.y, acc.y));
+    } else {
+        cfma(acc, a, b);
+    }
+}
+
+// CONJ: the second factor is conjugated; a conjugated first factor is the
+// conjugate of the product with the second one's conjugation flipped.
+template <int TM, int TN, int KS, bool CONJ, bool GATHER>
+__global__ void __launch_bounds__(256, 2) cgemm_kernel(const __grid_constant__ GemmLaunch gl) {
+    constexpr int KC = KS > 1 ? 16 : 8;                       // K of a chunk
+    constexpr int ST = 4;                                     // chunks in shared memory
+    constexpr int GT = 256 / KS;                              // threads of a group
+    constexpr int XN = TN / 4, XM = TM / 4;
+    constexpr int NA = TM * KC / 256, NB = TN * KC / 256;     // loads a thread and chunk
+    static_assert(XN * XM == GT, "4 x 4 outputs a thread");
+    constexpr int BUF = KC * (TM + 1 + TN + 1);
+    __shared__ __align__(16) cf sm[ST * BUF];
+    static_assert((KS - 1) * TM * TN <= ST * BUF, "the groups' sums fit");
+    GemmArgs g = gl.p[gl.two && blockIdx.z ? 1 : 0];
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+    if (m0 >= g.M || n0 >= g.N) return;
+    if (!gl.two) {
+        g.A += blockIdx.z * g.bsa;
+        g.B += blockIdx.z * g.bsb;
+        g.C += blockIdx.z * g.bsc;
+    }
+    if (GATHER) {
+        const int x = gl.ga.digit[blockIdx.y];
+        if (x < 0) return;
+        if (x >= gl.ga.ndig) g.K = 0;
+        else g.B += x * gl.ga.bdig;
+    }
+    const int tid = threadIdx.x, grp = tid / GT, t = tid % GT, tx = t % XN, ty = t / XN;
+    // this thread's elements of a chunk, along the unit stride of each operand:
+    // source (of chunk 0), K index (beyond K for an absent row or column)
+    const bool a_kfast = g.sak == 1, b_nfast = g.sbn == 1;
+    int ak[NA], bk[NB];
+    uint32_t ad[NA], bd[NB];
+    const cf* ap[NA];
+    const cf* bp[NB];
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+#pragma unroll
+    for (int q = 0; q < NA; ++q) {
+        const int e = tid + 256 * q;
+        const int k = a_kfast ? e % KC : e / TM, r = a_kfast ? e / KC : e % TM;
+        int row = m0 + r;
+        bool in = row < g.M;
+        if (GATHER && in) {
+            row = gl.ga.rows[row];
+            in = row >= 0;
+        }
+        ak[q] = in ? k : INT_MAX;
+        ad[q] = base + (k * (TM + 1) + r) * (uint32_t)sizeof(cf);
+        ap[q] = in ? g.A + row * g.sam + k * g.sak : g.A;
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int e = tid + 256 * q;
+        const int k = b_nfast ? e / TN : e % KC, c = b_nfast ? e % TN : e / KC;
+        const int col = n0 + c;
+        bk[q] = col < g.N ? k : INT_MAX;
+        bd[q] = base + (KC * (TM + 1) + k * (TN + 1) + c) * (uint32_t)sizeof(cf);
+        bp[q] = col < g.N ? g.B + k * g.sbk + col * g.sbn : g.B;
+    }
+    const long long da = KC * g.sak, db = KC * g.sbk;
+    const int chunks = (g.K + KC - 1) / KC;
+    // chunk c into buffer c mod ST by 8-byte asynchronous copies (zeros past K)
+    const auto fetch = [&](int c) {
+        if (c < chunks) {
+            const int left = g.K - c * KC;
+            const uint32_t off = (uint32_t)((c & (ST - 1)) * BUF) * (uint32_t)sizeof(cf);
+#pragma unroll
+            for (int q = 0; q < NA; ++q) {
+                const bool in = ak[q] < left;
+                copy8_async(ad[q] + off, in ? ap[q] : g.A, in ? 8u : 0u);
+                ap[q] += da;
+            }
+#pragma unroll
+            for (int q = 0; q < NB; ++q) {
+                const bool in = bk[q] < left;
+                copy8_async(bd[q] + off, in ? bp[q] : g.B, in ? 8u : 0u);
+                bp[q] += db;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     cf acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = cmake(0.f, 0.f);
-    const bool a_kfast = g.sak == 1;
-    const bool b_nfast = g.sbn == 1;
-    for (int k0 = 0; k0 < g.K; k0 += 16) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int idx = tid + q * 256;
-            int kk, tr;
-            if (a_kfast) { kk = idx & 15; tr = idx >> 4; } else { tr = idx & 63; kk = idx >> 6; }
-            const int row = m0 + tr, k = k0 + kk;
-            cf v = cmake(0.f, 0.f);
-            if (row < g.M && k < g.K) {
-                v = g.A[row * g.sam + k * g.sak];
-                if (g.conjA) v = cconj(v);
-            }
-            As[kk][tr] = v;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int idx = tid + q * 256;
-            int kk, tc;
-            if (b_nfast) { tc = idx & 63; kk = idx >> 6; } else { kk = idx & 15; tc = idx >> 4; }
-            const int col = n0 + tc, k = k0 + kk;
-            cf v = cmake(0.f, 0.f);
-            if (col < g.N && k < g.K) {
-                v = g.B[k * g.sbk + col * g.sbn];
-                if (g.conjB) v = cconj(v);
-            }
-            Bs[kk][tc] = v;
-        }
+    for (int c = 0; c < ST - 1; ++c) fetch(c);
+    for (int c = 0; c < chunks; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
         __syncthreads();
+        fetch(c + ST - 1);
+        const cf* As = sm + (c & (ST - 1)) * BUF;
+        const cf* Bs = As + KC * (TM + 1);
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
+        for (int kk = 0; kk < KC / KS; ++kk) {
+            const int k = kk * KS + grp;
             cf av[4], bv[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = As[kk][ty + 16 * i];
+            for (int i = 0; i < 4; ++i) av[i] = As[k * (TM + 1) + ty + XM * i];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx + 16 * j];
+            for (int j = 0; j < 4; ++j) bv[j] = Bs[k * (TN + 1) + tx + XN * j];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) cfma(acc[i][j], av[i], bv[j]);
+                for (int j = 0; j < 4; ++j) cfma_op<CONJ>(acc[i][j], av[i], bv[j]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (KS > 1) {
+        if (grp > 0) {
+            cf* dst = sm + (size_t)(grp - 1) * TM * TN;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dst[(4 * i + j) * GT + t] = acc[i][j];
         }
         __syncthreads();
+        if (grp > 0) return;
+#pragma unroll
+        for (int q = 0; q < KS - 1; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    acc[i][j] = cadd(acc[i][j], sm[(size_t)q * TM * TN + (4 * i + j) * GT + t]);
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
+        int row = m0 + ty + XM * i;
+        if (row >= g.M) continue;
+        if (GATHER) {
+            row = gl.ga.rows[row];
+            if (row < 0) continue;
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int row = m0 + ty + 16 * i, col = n0 + tx + 16 * j;
-            if (row < g.M && col < g.N) g.C[row * g.scm + col * g.scn] = acc[i][j];
+            const int col = n0 + tx + XN * j;
+            if (col < g.N)
+                g.C[row * g.scm + col * g.scn] = g.conjA ? cconj(acc[i][j]) : acc[i][j];
         }
+    }
+}
+
+// 64 x 64 tiles once they give every SM a CTA, else 32 x 32 (four times the tiles,
+// the K loop split over four groups of threads).  Measured with each: 64 steps
+// of two 256 x 512 x 256 products (64 large tiles), 2.64 ms small against 5.00
+// large; 64 products of 4096 x 256 x 256 (256 large tiles), 3.13 against 3.05.
+constexpr int kGemmSms = 152;
+
+bool small_tiles(long long m, long long n, long long count) {
+    return ((m + 63) / 64) * ((n + 63) / 64) * count < kGemmSms;
+}
+
+int cgemm_launch(const GemmLaunch& gl, int m, int n, int z, cudaStream_t s) {
+    const bool small = small_tiles(m, n, z);
+    const int t = small ? 32 : 64;
+    const dim3 grid((n + t - 1) / t, (m + t - 1) / t, z);
+    if (grid.y > 65535) return fail(MPS_ERR_ARG, "cgemm: too many rows");
+    if (grid.z > 65535) return fail(MPS_ERR_ARG, "cgemm: batch above 65535");
+    const bool conj = gl.p[0].conjA != gl.p[0].conjB;
+    if (small) {
+        if (conj) cgemm_kernel<32, 32, 4, true, false><<<grid, 256, 0, s>>>(gl);
+        else cgemm_kernel<32, 32, 4, false, false><<<grid, 256, 0, s>>>(gl);
+    } else {
+        if (conj) cgemm_kernel<64, 64, 1, true, false><<<grid, 256, 0, s>>>(gl);
+        else cgemm_kernel<64, 64, 1, false, false><<<grid, 256, 0, s>>>(gl);
+    }
+    MPS_LAUNCH_CHECK("cgemm_kernel");
+    return MPS_OK;
 }
 
 int cgemm(const GemmArgs& a, cudaStream_t s) {
     if (a.M <= 0 || a.N <= 0 || a.batch < 0) return MPS_OK;
-    dim3 grid((a.N + 63) / 64, (a.M + 63) / 64, a.batch > 1 ? a.batch : 1);
-    if (grid.y > 65535) return fail(MPS_ERR_ARG, "cgemm: too many rows");
-    if (grid.z > 65535) return fail(MPS_ERR_ARG, "cgemm: batch above 65535");
-    cgemm_kernel<<<grid, 256, 0, s>>>(a);
-    MPS_LAUNCH_CHECK("cgemm_kernel");
-    return MPS_OK;
+    GemmLaunch gl{};
+    gl.p[0] = a;
+    return cgemm_launch(gl, a.M, a.N, a.batch > 1 ? a.batch : 1, s);
+}
+
+// Two independent products in one launch (either may be empty).
+int cgemm2(const GemmArgs& a, const GemmArgs& b, cudaStream_t s) {
+    const bool ea = a.M <= 0 || a.N <= 0, eb = b.M <= 0 || b.N <= 0;
+    if (ea) return cgemm(b, s);
+    if (eb) return cgemm(a, s);
+    if ((a.conjA != a.conjB) != (b.conjA != b.conjB)) {
+        if (int rc = cgemm(a, s)) return rc;
+        return cgemm(b, s);
+    }
+    GemmLaunch gl{};
+    gl.p[0] = a;
+    gl.p[1] = b;
+    gl.two = 1;
+    return cgemm_launch(gl, max(a.M, b.M), max(a.N, b.N), 2, s);
+}
+
+// ---------------------------------------------------------------------------
+// Sampled amplitudes: a site's digit picks which of its d matrices multiplies
+// a bitstring's environment, so the bitstrings are grouped by digit, each
+// group padded to whole row tiles, and only the matrix picked is multiplied.
+// One block per site lists them: rows[site][...] (order kept within a digit),
+// one digit per tile (digits outside 0..d-1, whose amplitude is zero, come last
+// as digit d; -1: no tile).
+constexpr int kGroupT = 256;
+
+__global__ void __launch_bounds__(kGroupT) group_bits_kernel(const int8_t* __restrict__ bits,
+                                                             int nbits, int n, int d, int tile,
+                                                             int tiles, int* __restrict__ rows,
+                                                             int* __restrict__ digit) {
+    __shared__ int s_warp[kGroupT / 32];
+    const int site = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int* r = rows + (size_t)site * tiles * tile;
+    int* g = digit + (size_t)site * tiles;
+    int at = 0;                               // next free position, a multiple of tile
+    for (int x = 0; x <= d; ++x) {
+        int count = 0;
+        for (int s0 = 0; s0 < nbits; s0 += kGroupT) {
+            const int sidx = s0 + tid;
+            bool mine = false;
+            if (sidx < nbits) {
+                const int v = bits[(size_t)sidx * n + site];
+                mine = x < d ? v == x : (v < 0 || v >= d);
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, mine);
+            if (lane == 0) s_warp[warp] = __popc(mask);
+            __syncthreads();
+            int before = 0, all = 0;
+            for (int w = 0; w < kGroupT / 32; ++w) {
+                if (w < warp) before += s_warp[w];
+                all += s_warp[w];
+            }
+            if (mine) r[at + count + before + __popc(mask & ((1u << lane) - 1u))] = sidx;
+            count += all;
+            __syncthreads();
+        }
+        const int end = at + (count + tile - 1) / tile * tile;
+        for (int q = at + count + tid; q < end; q += kGroupT) r[q] = -1;
+        for (int q = at / tile + tid; q < end / tile; q += kGroupT) g[q] = x;
+        at = end;
+    }
+    for (int q = at / tile + tid; q < tiles; q += kGroupT) g[q] = -1;
 }
 
 // env'[s, r] = full[s, x_s * chir + r]
@@ -276,19 +491,33 @@ __global__ void select_kernel(const cf* __restrict__ full, cf* __restrict__ env,
     }
 }
 
-// probs[x] = Re sum_{l, r} conj(A[l, x, r]) W[l, x, r]: block x, FP64 sum.
-__global__ void __launch_bounds__(256) marginal_kernel(const cf* __restrict__ A,
-                                                       const cf* __restrict__ W, int chil,
-                                                       int d, int chir, float* __restrict__ probs) {
+// What the two directions of a marginal sweep leave for one site.
+struct MarginalSite {
+    const cf* T;                // T[l, x, r'] = sum_l' L[l, l'] conj(A[l', x, r'])
+    const cf* V;                // V[l, x, r'] = sum_r  conj(A[l, x, r]) R[r', r]
+    int chil, chir;
+};
+constexpr int kMarginalBatch = 64;
+struct MarginalArgs {
+    MarginalSite s[kMarginalBatch];
+};
+
+// probs[site * d + x] = Re sum_{l, r'} T[l, x, r'] conj(V[l, x, r']): block (x, site),
+// FP64 sum.
+__global__ void __launch_bounds__(256) marginal_kernel(const __grid_constant__ MarginalArgs a, int d,
+                                                       float* __restrict__ probs) {
     __shared__ double part[256];
     const int x = blockIdx.x;
-    const size_t total = (size_t)chil * chir;
+    const MarginalSite& s = a.s[blockIdx.y];
+    const int chir = s.chir, rows = s.chil;
     double acc = 0.0;
-    for (size_t t = threadIdx.x; t < total; t += blockDim.x) {
-        const size_t l = t / chir, r = t % chir;
-        const size_t o = (l * d + x) * chir + r;
-        const cf a = A[o], w = W[o];
-        acc += (double)a.x * w.x + (double)a.y * w.y;
+    // 8 warps take rows l in turn, lanes consecutive r'
+    for (int l = threadIdx.x >> 5; l < rows; l += 8) {
+        const size_t o = ((size_t)l * d + x) * chir;
+        for (int r = threadIdx.x & 31; r < chir; r += 32) {
+            const cf t = s.T[o + r], v = s.V[o + r];
+            acc += (double)t.x * v.x + (double)t.y * v.y;
+        }
     }
     part[threadIdx.x] = acc;
     __syncthreads();
@@ -296,7 +525,33 @@ __global__ void __launch_bounds__(256) marginal_kernel(const cf* __restrict__ A,
         if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) probs[x] = (float)part[0];
+    if (threadIdx.x == 0) probs[(size_t)blockIdx.y * d + x] = (float)part[0];
+}
+
+// sum_i a[i] b[i] in FP64 (one block) into out (re, im).
+__global__ void __launch_bounds__(1024) dot_kernel(const cf* __restrict__ a, const cf* __restrict__ b,
+                                                   size_t count, double* __restrict__ out) {
+    __shared__ double pr[1024], pi[1024];
+    double re = 0.0, im = 0.0;
+    for (size_t t = threadIdx.x; t < count; t += 1024) {
+        const cf x = a[t], y = b[t];
+        re += (double)x.x * y.x - (double)x.y * y.y;
+        im += (double)x.x * y.y + (double)x.y * y.x;
+    }
+    pr[threadIdx.x] = re;
+    pi[threadIdx.x] = im;
+    __syncthreads();
+    for (int o = 512; o > 0; o >>= 1) {
+        if (threadIdx.x < o) {
+            pr[threadIdx.x] += pr[threadIdx.x + o];
+            pi[threadIdx.x] += pi[threadIdx.x + o];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        out[0] = pr[0];
+        out[1] = pi[0];
+    }
 }
 
 __global__ void fill_one_kernel(cf* x, size_t count) {
@@ -373,8 +628,8 @@ extern "C" int mps_scale(void* stream, mps_c64* site, size_t count, float alpha_
 
 extern "C" size_t mps_sweep_workspace_bytes(int max_chi, int d) {
     if (max_chi < 1) max_chi = 1;
-    const size_t c = (size_t)max_chi;
-    return align_up((2 * c * c + (size_t)d * c * c) * sizeof(cf) + 1024, 256);
+    const size_t c = (size_t)max_chi;        // two environments and a product, for each direction
+    return align_up(2 * (2 * c * c + (size_t)d * c * c) * sizeof(cf) + 1024, 256);
 }
 
 extern "C" int mps_inner_product(void* stream, const mps_c64* const* a_sites, const int* chis_a,
@@ -389,35 +644,60 @@ extern "C" int mps_inner_product(void* stream, const mps_c64* const* a_sites, co
     for (int i = 0; i <= n; ++i) maxchi = max(maxchi, max(chis_a[i], chis_b[i]));
     if (workspace_bytes < mps_sweep_workspace_bytes(maxchi, d) || !workspace)
         return fail(MPS_ERR_WORKSPACE, "mps_inner_product: workspace too small");
+    // The left half of the chain is contracted from the left and the right half
+    // from the right, side by side: half the dependent steps, twice the work
+    // in each.  The two environments meet at the middle bond.
     const size_t cc = (size_t)maxchi * maxchi;
-    cf* E0 = static_cast<cf*>(workspace);
-    cf* E1 = E0 + cc;
-    cf* T = E1 + cc;
-    fill_one_kernel<<<1, 32, 0, s>>>(E0, 1);
+    double* dot = static_cast<double*>(workspace);
+    cf* E[2] = {reinterpret_cast<cf*>(dot + 2), nullptr};
+    E[1] = E[0] + cc;
+    cf* R[2] = {E[1] + cc, E[1] + 2 * cc};
+    cf* T = R[1] + cc;
+    cf* V = T + (size_t)d * cc;
+    fill_one_kernel<<<1, 32, 0, s>>>(E[0], 1);
     MPS_LAUNCH_CHECK("fill_one_kernel");
-    for (int i = 0; i < n; ++i) {
-        const int al = chis_a[i], ar = chis_a[i + 1], bl = chis_b[i], br = chis_b[i + 1];
-        const cf* A = reinterpret_cast<const cf*>(a_sites[i]);
-        const cf* B = reinterpret_cast<const cf*>(b_sites[i]);
-        // T[l, (x, r')] = sum_l' E[l, l'] conj(B[l', x, r'])
-        GemmArgs g1{al, d * br, bl, E0, bl, 1, 0, B, (long long)d * br, 1, 1, T, (long long)d * br, 1};
-        int rc = cgemm(g1, s);
-        if (rc) return rc;
-        // E'[r, r'] = sum_(l,x) A[(l,x), r] T[(l,x), r']
-        GemmArgs g2{ar, br, al * d, A, 1, ar, 0, T, br, 1, 0, E1, br, 1};
-        if (ar > 0 && br > 0 && al * d == 0) {
-            MPS_CUDA_CHECK(cudaMemsetAsync(E1, 0, (size_t)ar * br * sizeof(cf), s));
-        } else {
-            rc = cgemm(g2, s);
-            if (rc) return rc;
+    fill_one_kernel<<<1, 32, 0, s>>>(R[0], 1);
+    MPS_LAUNCH_CHECK("fill_one_kernel");
+    const int mid = n / 2;
+    const GemmArgs none{};
+    int ce = 0, cr = 0;
+    for (int t = 0; t < n - mid; ++t) {
+        GemmArgs l1 = none, l2 = none, r1 = none, r2 = none;
+        if (t < mid) {
+            const int al = chis_a[t], ar = chis_a[t + 1], bl = chis_b[t], br = chis_b[t + 1];
+            const cf* A = reinterpret_cast<const cf*>(a_sites[t]);
+            const cf* B = reinterpret_cast<const cf*>(b_sites[t]);
+            // T[l, (x, r')] = sum_l' E[l, l'] conj(B[l', x, r'])
+            l1 = GemmArgs{al, d * br, bl, E[ce], bl, 1, 0, B, (long long)d * br, 1, 1,
+                          T, (long long)d * br, 1};
+            // E'[r, r'] = sum_(l,x) A[(l,x), r] T[(l,x), r']
+            l2 = GemmArgs{ar, br, al * d, A, 1, ar, 0, T, br, 1, 0, E[ce ^ 1], br, 1};
+            ce ^= 1;
         }
-        cf* t = E0; E0 = E1; E1 = t;
+        {
+            const int i = n - 1 - t;
+            const int al = chis_a[i], ar = chis_a[i + 1], bl = chis_b[i], br = chis_b[i + 1];
+            const cf* A = reinterpret_cast<const cf*>(a_sites[i]);
+            const cf* B = reinterpret_cast<const cf*>(b_sites[i]);
+            // V[(l', x), r] = sum_r' conj(B[(l', x), r']) R[r, r']
+            r1 = GemmArgs{bl * d, ar, br, B, br, 1, 1, R[cr], 1, br, 0, V, ar, 1};
+            // R'[l, l'] = sum_(x,r) A[l, (x, r)] V[l', (x, r)]
+            r2 = GemmArgs{al, bl, d * ar, A, (long long)d * ar, 1, 0, V, 1, (long long)d * ar, 0,
+                          R[cr ^ 1], bl, 1};
+            cr ^= 1;
+        }
+        int rc = cgemm2(l1, r1, s);
+        if (rc) return rc;
+        rc = cgemm2(l2, r2, s);
+        if (rc) return rc;
     }
-    float2 res;
-    MPS_CUDA_CHECK(cudaMemcpyAsync(&res, E0, sizeof(float2), cudaMemcpyDeviceToHost, s));
+    dot_kernel<<<1, 1024, 0, s>>>(E[ce], R[cr], (size_t)chis_a[mid] * chis_b[mid], dot);
+    MPS_LAUNCH_CHECK("dot_kernel");
+    double res[2];
+    MPS_CUDA_CHECK(cudaMemcpyAsync(res, dot, sizeof(res), cudaMemcpyDeviceToHost, s));
     MPS_CUDA_CHECK(cudaStreamSynchronize(s));
-    result_host[0] = res.x;
-    result_host[1] = res.y;
+    result_host[0] = res[0];
+    result_host[1] = res[1];
     return MPS_OK;
 }
 
@@ -467,6 +747,28 @@ extern "C" int mps_wavefunction(void* stream, const mps_c64* const* sites, const
     return MPS_OK;
 }
 
+namespace {
+
+// Row tile of the grouped amplitude products: 64 where such tiles fill the GPU.
+int amplitude_tile(int nbits, int maxchi, int d) {
+    (void)d;
+    return small_tiles(nbits, maxchi, 1) ? 32 : 64;
+}
+int amplitude_tiles(int nbits, int d, int tile) { return (nbits + tile - 1) / tile + d + 1; }
+size_t amplitude_bytes(int nbits, int maxchi, int n, int d) {
+    const int tile = amplitude_tile(nbits, maxchi, d);
+    const size_t tiles = (size_t)amplitude_tiles(nbits, d, tile);
+    return 2 * (size_t)nbits * maxchi * sizeof(cf) + (size_t)n * tiles * (tile + 1) * sizeof(int);
+}
+
+}  // namespace
+
+extern "C" size_t mps_amplitudes_workspace_bytes(int nbits, int max_chi, int n, int d) {
+    if (nbits < 1 || max_chi < 1 || n < 1 || d < 1) return 0;
+    const size_t ungrouped = ((size_t)nbits * d * max_chi + 2 * (size_t)nbits * max_chi) * sizeof(cf);
+    return max(ungrouped, amplitude_bytes(nbits, max_chi, n, d));
+}
+
 extern "C" int mps_amplitudes(void* stream, const mps_c64* const* sites, const int* chis, int n,
                               int d, const int8_t* bits_dev, int nbits, mps_c64* out_dev,
                               void* workspace, size_t workspace_bytes) {
@@ -479,6 +781,35 @@ extern "C" int mps_amplitudes(void* stream, const mps_c64* const* sites, const i
     const size_t full_sz = (size_t)nbits * d * maxchi, env_sz = (size_t)nbits * maxchi;
     if (!workspace || workspace_bytes < (full_sz + 2 * env_sz) * sizeof(cf))
         return fail(MPS_ERR_WORKSPACE, "mps_amplitudes: workspace too small");
+    const int tile = amplitude_tile(nbits, maxchi, d);
+    if (workspace_bytes >= amplitude_bytes(nbits, maxchi, n, d) &&
+        amplitude_tiles(nbits, d, tile) <= 65535) {
+        cf* ge[2] = {static_cast<cf*>(workspace), static_cast<cf*>(workspace) + env_sz};
+        const int tiles = amplitude_tiles(nbits, d, tile);
+        int* rows = reinterpret_cast<int*>(ge[1] + env_sz);
+        int* digit = rows + (size_t)n * tiles * tile;
+        fill_one_kernel<<<grid_for(nbits), 256, 0, s>>>(ge[0], nbits);
+        MPS_LAUNCH_CHECK("fill_one_kernel");
+        group_bits_kernel<<<n, kGroupT, 0, s>>>(bits_dev, nbits, n, d, tile, tiles, rows, digit);
+        MPS_LAUNCH_CHECK("group_bits_kernel");
+        for (int i = 0, at = 0; i < n; ++i, at ^= 1) {
+            const int cl = chis[i], cr = chis[i + 1];
+            if (cr == 0) continue;
+            cf* dst = (i == n - 1) ? reinterpret_cast<cf*>(out_dev) : ge[at ^ 1];
+            GemmLaunch gl{};
+            gl.p[0] = GemmArgs{tiles * tile, cr, cl, ge[at], cl, 1, 0,
+                               reinterpret_cast<const cf*>(sites[i]), (long long)d * cr, 1, 0,
+                               dst, cr, 1};
+            gl.ga = GemmGather{rows + (size_t)i * tiles * tile, digit + (size_t)i * tiles, cr, d};
+            const dim3 grid((cr + tile - 1) / tile, tiles);
+            if (tile == 32) cgemm_kernel<32, 32, 4, false, true><<<grid, 256, 0, s>>>(gl);
+            else cgemm_kernel<64, 64, 1, false, true><<<grid, 256, 0, s>>>(gl);
+            MPS_LAUNCH_CHECK("cgemm_kernel");
+        }
+        return MPS_OK;
+    }
+    // a workspace without room for the groups: every digit's product, then the
+    // one picked
     cf* full = static_cast<cf*>(workspace);
     cf* env[2] = {full + full_sz, full + full_sz + env_sz};
     fill_one_kernel<<<grid_for(nbits), 256, 0, s>>>(env[0], nbits);
@@ -516,12 +847,22 @@ extern "C" int mps_cgemm(void* stream, int m, int n, int k, const mps_c64* a, lo
     return cgemm(g, s);
 }
 
+namespace {
+
+// Elements of the products T_i and U_i of every site (each 16-byte aligned).
+size_t marginal_cells(const int* chis, int n, int d) {
+    size_t cells = 0;
+    for (int i = 0; i < n; ++i) cells += align_up((size_t)chis[i] * d * chis[i + 1], 2);
+    return cells;
+}
+
+}  // namespace
+
 extern "C" size_t mps_marginals_workspace_bytes(const int* chis, int n, int d) {
     if (!chis || n < 1 || d < 1) return 0;
-    size_t envs = 0, maxchi = 1;
-    for (int i = 0; i < n; ++i) envs += (size_t)chis[i] * chis[i];
+    size_t maxchi = 1;
     for (int i = 0; i <= n; ++i) maxchi = max(maxchi, (size_t)chis[i]);
-    const size_t cells = envs + 2 * maxchi * maxchi + 2 * maxchi * d * maxchi;
+    const size_t cells = 2 * marginal_cells(chis, n, d) + 4 * maxchi * maxchi;
     return align_up(cells * sizeof(cf) + (size_t)n * d * sizeof(float) + 1024, 256);
 }
 
@@ -536,69 +877,52 @@ extern "C" int mps_site_marginals(void* stream, const mps_c64* const* sites, con
         return fail(MPS_ERR_WORKSPACE, "mps_site_marginals: workspace too small");
     size_t maxchi = 1;
     for (int i = 0; i <= n; ++i) maxchi = max(maxchi, (size_t)chis[i]);
-    // left environments L_i (ket, bra), i = 0..n-1, packed
-    cf* base = static_cast<cf*>(workspace);
-    size_t off = 0;
-    cf* R[2];
-    cf* U;
-    cf* W;
-    {
-        size_t envs = 0;
-        for (int i = 0; i < n; ++i) envs += (size_t)chis[i] * chis[i];
-        R[0] = base + envs;
-        R[1] = R[0] + maxchi * maxchi;
-        U = R[1] + maxchi * maxchi;
-        W = U + maxchi * d * maxchi;
-    }
-    float* probs_dev = reinterpret_cast<float*>(W + maxchi * d * maxchi);
-    fill_one_kernel<<<1, 32, 0, s>>>(base, 1);
+    // p_i(x) = sum L_i[l,l'] A[l,x,r] conj(A[l',x,r']) R_i[r,r']: the sweep from
+    // the left forms L A* at every site on its way and the one from the right the
+    // conjugate of A R (R is Hermitian), and their elementwise product is all
+    // that is left to sum.  The two sweeps run side by side, a product of each
+    // in a launch.
+    const size_t cc = maxchi * maxchi;
+    cf* L[2] = {static_cast<cf*>(workspace), static_cast<cf*>(workspace) + cc};
+    cf* R[2] = {L[1] + cc, L[1] + 2 * cc};
+    cf* T = R[1] + cc;
+    cf* V = T + marginal_cells(chis, n, d);
+    float* probs_dev = reinterpret_cast<float*>(V + marginal_cells(chis, n, d));
+    fill_one_kernel<<<1, 32, 0, s>>>(L[0], 1);
     MPS_LAUNCH_CHECK("fill_one_kernel");
-    for (int i = 0; i + 1 < n; ++i) {
-        const int cl = chis[i], cr = chis[i + 1];
-        const cf* A = reinterpret_cast<const cf*>(sites[i]);
-        cf* L = base + off;
-        cf* Ln = L + (size_t)cl * cl;
-        // U[l, (x, r')] = sum_l' L[l, l'] conj(A[l', x, r'])
-        GemmArgs g1{cl, d * cr, cl, L, cl, 1, 0, A, (long long)d * cr, 1, 1, U, (long long)d * cr, 1};
-        int rc = cgemm(g1, s);
-        if (rc) return rc;
-        // L'[r, r'] = sum_(l,x) A[(l,x), r] U[(l,x), r']
-        if (cr > 0 && cl == 0) {
-            MPS_CUDA_CHECK(cudaMemsetAsync(Ln, 0, (size_t)cr * cr * sizeof(cf), s));
-        } else {
-            GemmArgs g2{cr, cr, cl * d, A, 1, cr, 0, U, cr, 1, 0, Ln, cr, 1};
-            rc = cgemm(g2, s);
-            if (rc) return rc;
-        }
-        off += (size_t)cl * cl;
-    }
-    // right-to-left: p_i(x) = sum L_i[l,l'] A[l,x,r] conj(A[l',x,r']) R_i[r,r']
     fill_one_kernel<<<1, 32, 0, s>>>(R[0], 1);
     MPS_LAUNCH_CHECK("fill_one_kernel");
-    int cur = 0;
-    for (int i = n - 1; i >= 0; --i) {
-        const int cl = chis[i], cr = chis[i + 1];
+    std::vector<size_t> off(n + 1, 0);
+    for (int i = 0; i < n; ++i) off[i + 1] = off[i] + align_up((size_t)chis[i] * d * chis[i + 1], 2);
+    for (int t = 0; t < n; ++t) {
+        const int i = t, j = n - 1 - t, cur = t & 1;
+        const int il = chis[i], ir = chis[i + 1], jl = chis[j], jr = chis[j + 1];
         const cf* A = reinterpret_cast<const cf*>(sites[i]);
-        cf* L = base + off;
-        // U[(l, x), r'] = sum_r A[(l, x), r] R[r, r']
-        GemmArgs g1{cl * d, cr, cr, A, cr, 1, 0, R[cur], cr, 1, 0, U, cr, 1};
-        int rc = cgemm(g1, s);
+        const cf* B = reinterpret_cast<const cf*>(sites[j]);
+        cf* Ti = T + off[i];
+        cf* Vj = V + off[j];
+        // T[l, (x, r')] = sum_l' L[l, l'] conj(A[l', x, r']);  L'[r, r'] = A^T T
+        const GemmArgs l1{il, d * ir, il, L[cur], il, 1, 0, A, (long long)d * ir, 1, 1,
+                          Ti, (long long)d * ir, 1};
+        const GemmArgs l2{ir, ir, il * d, A, 1, ir, 0, Ti, ir, 1, 0, L[cur ^ 1], ir, 1};
+        // V[(l, x), r'] = sum_r conj(A[(l, x), r]) R[r', r];  R'[l, l'] = A V^T
+        const GemmArgs r1{jl * d, jr, jr, B, jr, 1, 1, R[cur], 1, jr, 0, Vj, jr, 1};
+        const GemmArgs r2{jl, jl, d * jr, B, (long long)d * jr, 1, 0, Vj, 1, (long long)d * jr, 0,
+                          R[cur ^ 1], jl, 1};
+        int rc = cgemm2(l1, r1, s);
         if (rc) return rc;
-        // W[l', (x, r')] = sum_l L[l, l'] U[l, (x, r')]
-        GemmArgs g2{cl, d * cr, cl, L, 1, cl, 0, U, (long long)d * cr, 1, 0, W, (long long)d * cr, 1};
-        rc = cgemm(g2, s);
-        if (rc) return rc;
-        marginal_kernel<<<d, 256, 0, s>>>(A, W, cl, d, cr, probs_dev + (size_t)i * d);
-        MPS_LAUNCH_CHECK("marginal_kernel");
-        if (i > 0) {
-            // R'[l, l'] = sum_(x, r') U[l, (x, r')] conj(A[l', (x, r')])
-            GemmArgs g3{cl, cl, d * cr, U, (long long)d * cr, 1, 0, A, 1, (long long)d * cr, 1,
-                        R[cur ^ 1], cl, 1};
-            rc = cgemm(g3, s);
+        if (t + 1 < n) {
+            rc = cgemm2(l2, r2, s);
             if (rc) return rc;
-            cur ^= 1;
-            off -= (size_t)chis[i - 1] * chis[i - 1];
         }
+    }
+    for (int i0 = 0; i0 < n; i0 += kMarginalBatch) {
+        MarginalArgs a{};
+        const int count = min(kMarginalBatch, n - i0);
+        for (int q = 0; q < count; ++q)
+            a.s[q] = MarginalSite{T + off[i0 + q], V + off[i0 + q], chis[i0 + q], chis[i0 + q + 1]};
+        marginal_kernel<<<dim3(d, count), 256, 0, s>>>(a, d, probs_dev + (size_t)i0 * d);
+        MPS_LAUNCH_CHECK("marginal_kernel");
     }
     MPS_CUDA_CHECK(cudaMemcpyAsync(probs_host, probs_dev, (size_t)n * d * sizeof(float),
                                    cudaMemcpyDeviceToHost, s));

@@ -1,5 +1,5 @@
-// Jacobi rotation parameters shared by the FP32 SIMT sweep kernel
-// (jacobi.cu) and the tensor-core block sweep (tcjacobi.cu).
+// Jacobi rotation parameters shared by the FP32 SIMT sweep kernels (jacobi.cu,
+// gramsweep.cu) and the tensor-core block sweep (tcjacobi.cu).
 #pragma once
 
 #include "common.cuh"
@@ -82,4 +82,65 @@ __device__ __forceinline__ void apply_rot(const Rot& r, cf& x, cf& q) {
     q = cmake(nqr, nqi);
 }
 
+// The same rotation for the two-sided steps on a Gram matrix (one pair a lane,
+// where the chain of dependent operations is what a step waits for): tp, sigma
+// and dn from one chain of three approximate reciprocals: with u = 1 / sqrt(p^2 + 4
+// |gamma|^2), p = b - a, the double angle gives c^2 = (1 + |p| u) / 2 and
+// s = |gamma| u / c; tp = s^2 / (1 + c).  Both reciprocal square roots take a
+// Newton step, and tp comes from s^2, so a rotation changes no norm by more
+// than a few ulps of s^2.  A pair whose squared cosine is not above thr gets the
+// identity; in a careful visit (one with tiny columns), pairs whose squares could
+// leave FP32's range take the scaled form above.
+// Squared norms above this (theta's is in [1, 4)) keep every product that a
+// rotation is decided on within FP32's normal range.
+constexpr float kTinyNorm2 = 1e-9f;
+__device__ __forceinline__ float newton_rsqrt(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r * fmaf(-0.5f * x * r, r, 1.5f);
+}
+// 1 / x to about an ulp (x near 1).
+__device__ __forceinline__ float recip(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(fmaf(-x, r, 1.f), r, r);
+}
+struct PairRot {
+    float tp, sr, si, dn, c, ic;             // (c and 1 / c: 1 where it does not rotate)
+    bool rot;
+};
+__device__ __forceinline__ PairRot pair_rotation(float a, float b, cf gam, float thr,
+                                                 bool careful) {
+    const float g2 = cabs2(gam), ab = a * b, p = b - a;
+    const bool small = careful && (g2 < 1e-30f || ab < 1e-30f);
+    PairRot o;
+    o.rot = !small && g2 > thr * ab;
+    // (a pair of zero columns stays finite)
+    const float u = newton_rsqrt(fmaxf(fmaf(p, p, 4.f * g2), 1e-37f));
+    const float c2 = fmaf(0.5f * fabsf(p), u, 0.5f);
+    const float ic = newton_rsqrt(c2);
+    const float k = o.rot ? u * ic : 0.f;                // s = |gamma| k
+    const float ks = p >= 0.f ? k : -k;
+    float rc;
+    o.sr = ks * gam.x;
+    o.si = -ks * gam.y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(fmaf(c2, ic, 1.f)));
+    o.tp = g2 * k * k * rc;
+    o.dn = g2 * ks * ic;                                 // t |gamma| = s |gamma| / c
+    o.c = o.rot ? c2 * ic : 1.f;
+    o.ic = o.rot ? ic : 1.f;
+    if (careful) {
+        if (small && pair_cos2(gam, g2, a, b) > thr) {
+            const Rot r = make_rot(a, b, gam);
+            o.tp = r.tp;
+            o.sr = r.sigma.x;
+            o.si = r.sigma.y;
+            o.dn = r.dn;
+            o.c = 1.f - r.tp;
+            o.ic = recip(o.c);
+            o.rot = true;
+        }
+    }
+    return o;
+}
 }  // namespace mps

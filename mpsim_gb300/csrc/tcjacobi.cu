@@ -122,6 +122,7 @@ struct Aux {
     uint32_t tmem;
     int item, abort, skip;   // the claimed visit, the stop flag, its skip decision
     int rotated;          // some pair of this visit needs a rotation
+    int tiny;             // some column is too short for pair_rotation's fast form
     int col[TJ_W];        // physical column of each visit column (-1: zero padding)
     float diag[TJ_W];     // diagonal of G (squared column norms)
     cf gam[TJ_W];         // G[cP][cQ] of the 32 pairs of the next inner step (the ring
@@ -333,6 +334,7 @@ __device__ __forceinline__ bool visit(const TwoQGeom& g, int j, int I, int J, bo
     }
     if (tid == 0) {
         ax.rotated = 0;
+        ax.tiny = 0;
         ax.cmax = 0.f;
     }
     __syncthreads();
@@ -416,7 +418,9 @@ __device__ __forceinline__ bool visit(const TwoQGeom& g, int j, int I, int J, bo
     __syncthreads();
     if (tid < TJ_W) {
         G[gidx(tid, tid)].y = 0.f;
-        ax.diag[tid] = G[gidx(tid, tid)].x;
+        const float dg = G[gidx(tid, tid)].x;
+        ax.diag[tid] = dg;
+        if (dg > 0.f && dg < kTinyNorm2) ax.tiny = 1;
     }
     __syncthreads();
     const long long c1 = clock64();
@@ -449,6 +453,7 @@ __device__ __forceinline__ bool visit(const TwoQGeom& g, int j, int I, int J, bo
         __syncthreads();
     }
     const bool work = ax.rotated != 0;
+    const bool careful = ax.tiny != 0;
     const int nsteps = TJ_W - 1;           // the full visit's steps
     int rsteps = 0, rpairs = 0;
     if (work && !full) {
@@ -506,16 +511,13 @@ __device__ __forceinline__ bool visit(const TwoQGeom& g, int j, int I, int J, bo
             cf sg = cmake(0.f, 0.f);
             bool rot;
             {
-                const float a = dP, bb = dQ;
-                const cf gam = ax.gam[(b * 32) + lane];
-                rot = pair_cos2(gam, cabs2(gam), a, bb) > kInnerTol2 * tol2;
-                if (rot) {
-                    const Rot r = make_rot(a, bb, gam);
-                    tp = r.tp;
-                    sg = r.sigma;
-                    na = a - r.dn;
-                    nb = bb + r.dn;
-                }
+                const PairRot r = pair_rotation(dP, dQ, ax.gam[(b * 32) + lane],
+                                                kInnerTol2 * tol2, careful);
+                rot = r.rot;
+                tp = r.tp;
+                sg = cmake(r.sr, r.si);
+                na = dP - r.dn;
+                nb = dQ + r.dn;
             }
             const unsigned rmask = __ballot_sync(0xffffffffu, rot);
             if (rmask) {
@@ -543,10 +545,8 @@ __device__ __forceinline__ bool visit(const TwoQGeom& g, int j, int I, int J, bo
                     eQ[h].x = fmaf(mp, sg.x, fmaf(-mq, tp, eQ[h].x));
                     eQ[h].y = fmaf(-mp, sg.y, eQ[h].y);
                 }
-                if (rot) {
-                    dP = na;
-                    dQ = nb;
-                }
+                dP = na;
+                dQ = nb;
             }
             if (s + 1 < TJ_BC) {
                 // the Q columns move to the lane of their next pair
@@ -625,17 +625,13 @@ __device__ __forceinline__ bool visit(const TwoQGeom& g, int j, int I, int J, bo
             cf sg = cmake(0.f, 0.f);
             bool rot;
             {
-                const float a = dP, b = dQ;
-                const cf gam = ax.gam[lane];
                 // per-step rotation decision in FP32 (kInnerTol2 above)
-                rot = pair_cos2(gam, cabs2(gam), a, b) > kInnerTol2 * tol2;
-                if (rot) {
-                    const Rot r = make_rot(a, b, gam);
-                    tp = r.tp;
-                    sg = r.sigma;
-                    na = a - r.dn;        // the norm transfer of rot.cuh
-                    nb = b + r.dn;
-                }
+                const PairRot r = pair_rotation(dP, dQ, ax.gam[lane], kInnerTol2 * tol2, careful);
+                rot = r.rot;
+                tp = r.tp;
+                sg = cmake(r.sr, r.si);
+                na = dP - r.dn;           // the norm transfer of rot.cuh
+                nb = dQ + r.dn;
             }
             // every warp holds the same 32 decisions: a step without a
             // rotation changes nothing
@@ -652,10 +648,8 @@ __device__ __forceinline__ bool visit(const TwoQGeom& g, int j, int I, int J, bo
                     H[gidx(cQ, r)] = cconj(gQ[h]);
                 }
                 __syncthreads();
-                if (rot) {
-                    dP = na;
-                    dQ = nb;
-                }
+                dP = na;
+                dQ = nb;
                 // pass 2: G' = H^H R (= R^H G R) and E <- (I + E) R - I =
                 // E R + (R - I), whose identity part adds -tp, -sigma to
                 // column cP and conj(sigma), -tp to column cQ in rows cP, cQ.
