@@ -177,8 +177,9 @@ __global__ void scale_kernel(cf* __restrict__ x, size_t count, cf alpha, int con
 // different products in one launch (the two directions of a sweep).
 //
 // 256 threads form TM x TN outputs, 4 x 4 a thread (rows ty + TM/4 i, columns
-// tx + TN/4 j), from K chunks copied into shared memory three ahead; KS groups of threads each take a share of every chunk and are summed at
-// the end, so that a 32 x 32 tile keeps all eight warps busy.
+// tx + TN/4 j), from K chunks copied into shared memory three ahead; KS groups of
+// threads each take a share of every chunk and are summed at the end, so that a
+// 32 x 32 tile keeps all eight warps busy.
 //
 // What bounds it: the FP32 pipes for large products (64 x 64 tiles: 8 wavefronts
 // of shared-memory reads for 64 FMAs a thread), and the few tiles of the sweeps'

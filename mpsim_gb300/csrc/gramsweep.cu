@@ -910,7 +910,8 @@ gram_sweep_kernel(TwoQGeom g, float tol2, SweepSync sync, int tbase) {
 constexpr int GS_BEGIN_T = 512;
 
 __global__ void __launch_bounds__(GS_BEGIN_T)
-gram_begin_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs, SweepSync sync) {
+gram_begin_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs, SweepSync sync,
+                  GramBegin b) {
     __shared__ int s_warp[GS_BEGIN_T / 32];
     __shared__ int s_nb;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -919,7 +920,9 @@ gram_begin_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs, Sw
         g.counter[0] = 0;
         *sync.next_item = 0;
         if (g.tc_mode) g.counter[4] = g.counter[5] = 0;
-        else *sync.error = 0;
+        if (b.clear_error) *sync.error = 0;
+        // an expired wait also marks every job's status
+        else if (b.end_sweep && *sync.error) g.counter[3] = 1;
     }
     __syncthreads();
     int base = 0;
@@ -927,7 +930,15 @@ gram_begin_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs, Sw
         const int j = j0 + tid;
         bool live = false;
         int4 e = make_int4(j, 0, 0, 0);
-        if (j < njobs && !g.done[j]) {
+        bool open = j < njobs && !g.done[j];
+        if (open && b.end_sweep) {
+            if (!(g.offmax[j] > b.tol2)) {
+                g.done[j] = 1;
+                open = false;
+            }
+            g.offmax[j] = 0.f;
+        }
+        if (open) {
             const int m = jobs[j].chi_l * g.d, n = jobs[j].chi_r * g.d;
             const int lc = jobs[j].keep_left_canonical;
             e.y = max(m, n);
@@ -950,7 +961,17 @@ gram_begin_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs, Sw
         base += all;
         __syncthreads();
     }
-    if (tid == 0) g.gact[0] = make_int4(base, s_nb - 1, s_nb / 2, 0);
+    if (tid == 0) {
+        g.gact[0] = make_int4(base, s_nb - 1, s_nb / 2, 0);
+        if (b.record) {
+            volatile int* rec = b.record;
+            rec[0] = base;
+            rec[1] = g.counter[1];
+            rec[2] = *sync.error;
+            __threadfence_system();
+            rec[3] = b.seq;
+        }
+    }
 }
 
 template <int LW, int S, int NG, int NA>
@@ -985,8 +1006,8 @@ int launch(int njobs, int rounds, int pairs, const TwoQGeom& g, float tol2, cons
 }  // namespace
 
 int gram_begin_launch(const mps_2q_job* jobs, int njobs, const TwoQGeom& g, const SweepSync& sync,
-                      cudaStream_t s) {
-    gram_begin_kernel<<<1, GS_BEGIN_T, 0, s>>>(jobs, g, njobs, sync);
+                      const GramBegin& b, cudaStream_t s) {
+    gram_begin_kernel<<<1, GS_BEGIN_T, 0, s>>>(jobs, g, njobs, sync, b);
     MPS_LAUNCH_CHECK("gram_begin_kernel");
     return MPS_OK;
 }

@@ -674,9 +674,13 @@ __global__ void sweep_end_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g
     g.offmax[j] = 0.f;
 }
 
-__global__ void init_slots_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs) {
+__global__ void init_slots_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs,
+                                  int* stamps, size_t nstamps) {
     // V = identity for jobs that track V, identity column maps, bookkeeping
-    // cleared
+    // cleared, no block stamped (stamps: all of them, in one stretch)
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nstamps;
+         e += (size_t)gridDim.x * blockDim.x)
+        stamps[e] = -1;
     const size_t per = (size_t)g.cslot * g.cslot;
     const size_t total = per * njobs;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
@@ -697,6 +701,7 @@ __global__ void init_slots_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom 
         g.done[t] = 0;
         g.offmax[t] = 0.f;
         g.need[t] = 0;
+        g.nrm2[t] = 0.0;
     }
     if (t < 8) g.counter[t] = 0;
 }
@@ -1231,7 +1236,6 @@ __global__ void __launch_bounds__(256) unscale_kernel(const mps_2q_job* __restri
 }
 
 int scale_theta(const mps_2q_job* jobs, int njobs, const TwoQGeom& g, cudaStream_t s) {
-    MPS_CUDA_CHECK(cudaMemsetAsync(g.nrm2, 0, (size_t)njobs * sizeof(double), s));
     theta_norm_kernel<<<dim3((g.cslot + 7) / 8, njobs), 256, 0, s>>>(g);
     MPS_LAUNCH_CHECK("theta_norm_kernel");
     const size_t count = (size_t)g.lslot * g.cslot;
@@ -1427,7 +1431,26 @@ Layout make_layout(int njobs, int max_m, int max_n, bool pieces = false, bool gr
     return lo;
 }
 
+// Pinned host memory the device reports to: the values of a convergence read,
+// or a Gram sweep's record (jobs left, NaN count, expired waits, sequence
+// number), with the last sequence number this thread gave out.
 thread_local int* t_pinned = nullptr;
+thread_local int t_seq = 0;
+
+// Waits until the device has written record `seq`.
+int wait_record(const int* rec, int seq, cudaStream_t s) {
+    for (int spin = 0;; ++spin) {
+        if (__atomic_load_n(rec + 3, __ATOMIC_ACQUIRE) == seq) return MPS_OK;
+        if ((spin & 0xfff) != 0xfff) continue;
+        // an error on the stream, or a finished stream without the record,
+        // would otherwise be waited for for ever
+        const cudaError_t e = cudaStreamQuery(s);
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess) return cuda_fail(e, "waiting for a sweep");
+        if (__atomic_load_n(rec + 3, __ATOMIC_ACQUIRE) == seq) return MPS_OK;
+        return fail(MPS_ERR_CUDA, "mps_apply_2q_batch: a sweep left no record");
+    }
+}
 
 }  // namespace
 
@@ -1538,15 +1561,14 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
     sync.nbmax = lo.nbmax;
     sync.wait_limit = (params && params->wait_limit > 0) ? params->wait_limit : (1 << 22);
     sync.stall_test = params ? params->stall_test : 0;
-    // padding rows and columns of X must be zero; no block has a stamp yet
+    // padding rows and columns of X must be zero
     MPS_CUDA_CHECK(cudaMemsetAsync(g.X, 0, lo.off_V - lo.off_X, s));
-    MPS_CUDA_CHECK(cudaMemsetAsync(g.vstamp, 0xff, lo.off_qst - lo.off_vst +
-                                                       (size_t)njobs * lo.qstride * sizeof(int), s));
     {
         const size_t total = (size_t)njobs * lo.cslot * lo.cslot;
         int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
         blocks = max(blocks, (njobs + 255) / 256);
-        init_slots_kernel<<<blocks, 256, 0, s>>>(jobs, g, njobs);
+        const size_t nstamps = (lo.off_qst - lo.off_vst) / sizeof(int) + (size_t)njobs * lo.qstride;
+        init_slots_kernel<<<blocks, 256, 0, s>>>(jobs, g, njobs, g.vstamp, nstamps);
         MPS_LAUNCH_CHECK("init_slots_kernel");
         if (mixed) {
             count_simt_jobs_kernel<<<(njobs + 255) / 256, 256, 0, s>>>(jobs, d, njobs, g.counter);
@@ -1580,7 +1602,8 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
 
     if (!t_pinned && !capturing) {
         MPS_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&t_pinned), 8 * sizeof(int),
-                                     cudaHostAllocDefault));
+                                     cudaHostAllocPortable | cudaHostAllocMapped));
+        t_pinned[3] = 0;
     }
     int npow2 = 1;
     while (npow2 < lo.cslot) npow2 <<= 1;
@@ -1591,14 +1614,50 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
         // mixed calls: whether the last sweep left jobs for each sweep kernel
         // (unknown, so both run, before the first read and under capture)
         bool tc_left = true, simt_left = true;
-        for (sweeps = 1; sweeps <= max_sweeps; ++sweeps) {
+        // The plain form keeps a sweep queued while the host looks at the one
+        // before: sweep s's begin kernel also ends sweep s - 1 and writes the
+        // jobs left to the host's record, so nothing on the stream waits for the
+        // host (a sweep queued after the last one finds no job and returns).
+        // Per sweep of small jobs this took ~30 of ~75 us.
+        const bool piped = gram && !mixed && !capturing;
+        for (sweeps = 1; piped; ++sweeps) {
+            const int seq = ++t_seq;
+            rc = gram_begin_launch(jobs, njobs, g, sync, GramBegin{sweeps > 1, sweeps == 1, tol2,
+                                                                   t_pinned, seq}, s);
+            if (rc) return rc;
+            if (sweeps <= max_sweeps) {
+                if (cmax > 2 * bc) {
+                    presort_kernel<<<njobs, PRESORT_T, sort_smem, s>>>(jobs, g, npow2, bc,
+                                                                       sweeps * tbase_stride);
+                    MPS_LAUNCH_CHECK("presort_kernel");
+                }
+                rc = gram_sweep_launch(njobs, rounds, pairs, g, tol2, sync, sweeps * tbase_stride, s);
+                if (rc) return rc;
+            }
+            if (sweeps == 1) continue;
+            rc = wait_record(t_pinned, seq, s);
+            if (rc) return rc;
+            if (t_pinned[2] != 0) {
+                MPS_CUDA_CHECK(cudaStreamSynchronize(s));
+                return fail(MPS_ERR_TIMEOUT, "mps_apply_2q_batch: a round-dependency wait inside the "
+                                             "sweep kernel expired; results are invalid");
+            }
+            converged = t_pinned[0] == 0;
+            if (converged || sweeps > max_sweeps) {
+                --sweeps;
+                break;
+            }
+        }
+        for (sweeps = piped ? sweeps : 1; !piped && sweeps <= max_sweeps; ++sweeps) {
             if (cmax > 2 * bc) {
                 presort_kernel<<<njobs, PRESORT_T, sort_smem, s>>>(jobs, g, npow2, bc,
                                                                    sweeps * tbase_stride);
                 MPS_LAUNCH_CHECK("presort_kernel");
             }
             if (gram) {
-                if (int e = gram_begin_launch(jobs, njobs, g, sync, s)) return e;
+                rc = gram_begin_launch(jobs, njobs, g, sync, GramBegin{false, !mixed, tol2, nullptr, 0},
+                                       s);
+                if (rc) return rc;
             } else {
                 MPS_CUDA_CHECK(cudaMemsetAsync(g.counter, 0, sizeof(int), s));
                 if (mixed) MPS_CUDA_CHECK(cudaMemsetAsync(g.counter + 4, 0, 2 * sizeof(int), s));
@@ -1840,7 +1899,7 @@ extern "C" int mps_apply_2q_batch_noalloc(void* stream, const mps_2q_job* jobs, 
         const size_t total = (size_t)njobs * lo.cslot * lo.cslot;
         int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
         blocks = max(blocks, (njobs + 255) / 256);
-        init_slots_kernel<<<blocks, 256, 0, s>>>(jobs, g, njobs);
+        init_slots_kernel<<<blocks, 256, 0, s>>>(jobs, g, njobs, nullptr, 0);
         MPS_LAUNCH_CHECK("init_slots_kernel");
     }
     const int max_chil = (max_m + d - 1) / d, max_chir = (max_n + d - 1) / d;

@@ -108,10 +108,18 @@ int lq_precondition(const mps_2q_job* jobs, int njobs, int max_m, int max_n, con
 constexpr int kGramRows = 1024;
 constexpr int kGramBlock = 8;
 // gram_begin_launch, before each sweep, lists the jobs left in g.gact and clears
-// counter[0] (and [4], [5] of a mixed call), the item counter and, in the plain
-// form, the error word.
+// counter[0] (and [4], [5] of a mixed call) and the item counter; as asked it
+// first ends the sweep before (jobs without a pair over the tolerance are
+// done), clears the error word, and writes (jobs left, NaN count, error word,
+// seq) to a record in pinned host memory.
+struct GramBegin {
+    bool end_sweep, clear_error;
+    float tol2;
+    int* record;
+    int seq;
+};
 int gram_begin_launch(const mps_2q_job* jobs, int njobs, const TwoQGeom& g, const SweepSync& sync,
-                      cudaStream_t s);
+                      const GramBegin& b, cudaStream_t s);
 int gram_sweep_launch(int njobs, int rounds, int pairs, const TwoQGeom& g,
                       float tol2, const SweepSync& sync, int tbase, cudaStream_t s);
 
