@@ -351,6 +351,18 @@ class MPS:
                  *, track_norms: bool = False, record_svals: bool = False,
                  on_unconverged: str = "raise", precision: str = "plain",
                  autotune: bool = True) -> None:
+        self._setup(nqudits, qudit_dimension, tensor_prefix, track_norms, record_svals,
+                    on_unconverged, precision, autotune)
+        d = self._qudit_dimension
+        init = torch.zeros((self._nqudits, 1, d, 1), dtype=torch.complex64)
+        init[:, 0, 0, 0] = 1.0
+        init = init.to(self._device)
+        self._site_list = [init[i].clone() for i in range(self._nqudits)]
+
+    def _setup(self, nqudits, qudit_dimension=2, tensor_prefix="q", track_norms=False,
+               record_svals=False, on_unconverged="raise", precision="plain",
+               autotune=True) -> None:
+        """Everything of a new state but its sites."""
         if nqudits < 2:
             raise ValueError(f"Number of qudits must be greater than 2 but is {nqudits}.")
         self._nqudits = int(nqudits)
@@ -397,18 +409,19 @@ class MPS:
         # bumped whenever a site tensor is replaced; is_valid caches per value
         self._version = 0
         self._valid_at = (-1, False)
-        d = self._qudit_dimension
-        init = torch.zeros((self._nqudits, 1, d, 1), dtype=torch.complex64)
-        init[:, 0, 0, 0] = 1.0
-        init = init.to(self._device)
-        self._site_list = [init[i].clone() for i in range(self._nqudits)]
 
     @classmethod
     def from_sites(cls, sites, qudit_dimension: int, **kwargs) -> "MPS":
         """An MPS around existing device site tensors ((chi_l, d, chi_r)
         complex64, shared, not copied), e.g. a CircuitPlan's final state."""
         sites = list(sites)
-        mps = cls(len(sites), qudit_dimension, **kwargs)
+        if cls.__init__ is MPS.__init__:
+            # no product state that the given sites would replace (20 sites:
+            # 0.4 ms, most of what reading a circuit's state out of a plan took)
+            mps = cls.__new__(cls)
+            mps._setup(len(sites), qudit_dimension, **kwargs)
+        else:
+            mps = cls(len(sites), qudit_dimension, **kwargs)
         for t in sites:
             if t.dtype != torch.complex64 or t.dim() != 3 or int(t.shape[1]) != mps._qudit_dimension:
                 raise ValueError("sites must be (chi_l, d, chi_r) complex64 tensors")

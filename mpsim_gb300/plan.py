@@ -328,9 +328,9 @@ class CircuitPlan:
         every run or replay)."""
         d = self.d
         out = []
+        elements = self.arena.view(torch.complex64)
         for o, (cl, cr) in self._final[index]:
-            nbytes = cl * d * cr * 8
-            out.append(self.arena[o:o + nbytes].view(torch.complex64).view(cl, d, cr))
+            out.append(elements.as_strided((cl, d, cr), (d * cr, cr, 1), o // 8))
         return out
 
     def state(self, index: int, precision: Optional[str] = None) -> MPS:
