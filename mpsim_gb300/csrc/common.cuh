@@ -119,6 +119,9 @@ int cuda_fail(cudaError_t e, const char* what);
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// SMs of a GB300: tile sizes are chosen by how many tiles reach every SM.
+constexpr int kSms = 152;
+
 // Devices a process may use with this library (per-device one-time setup).
 constexpr int kMaxDevices = 64;
 

@@ -9,13 +9,12 @@
 //   renormalize / dagger   mpsim/core.py:567-594, 502-505
 //   marginals for sample   mpsim/core.py:655-667 (reduced_density_matrix(i)
 //                          diagonal, core.py:596-653)
-#include <limits.h>
-
 #include <atomic>
 #include <string>
 #include <vector>
 
 #include "common.cuh"
+#include "gemm.cuh"
 
 namespace mps {
 
@@ -176,13 +175,7 @@ __global__ void scale_kernel(cf* __restrict__ x, size_t count, cf alpha, int con
 // bsb, bsc between batches (zero: the same matrix for every batch), or two
 // different products in one launch (the two directions of a sweep).
 //
-// 256 threads form TM x TN outputs, 4 x 4 a thread (rows ty + TM/4 i, columns
-// tx + TN/4 j), from K chunks copied into shared memory three ahead; KS groups of
-// threads each take a share of every chunk and are summed at the end, so that a
-// 32 x 32 tile keeps all eight warps busy.
-//
-// What bounds it: the FP32 pipes for large products (64 x 64 tiles: 8 wavefronts
-// of shared-memory reads for 64 FMAs a thread), and the few tiles of the sweeps'
+// What bounds it: the FP32 pipes for large products (gemm.cuh), and the few tiles of the sweeps'
 // 256 x 512 x 256 steps otherwise -- there 32 x 32 tiles, and both directions
 // of a sweep in one launch, put work on every SM.  Measured (GB300) against one
 // direction at a time, 64 x 64 tiles and loads that were waited for chunk by
@@ -190,20 +183,6 @@ __global__ void scale_kernel(cf* __restrict__ x, size_t count, cf alpha, int con
 // 53% busy, 74% of issue slots), marginals of 48 sites of chi=128 8.1 -> 0.96 ms
 // (the third product a site is gone too), 4096 amplitudes at chi=256 7.6 -> 3.1 ms
 // (half of the products were of digits not asked for).
-struct GemmArgs {
-    int M, N, K;
-    const cf* A;
-    long long sam, sak;
-    int conjA;
-    const cf* B;
-    long long sbk, sbn;
-    int conjB;
-    cf* C;
-    long long scm, scn;
-    int batch;                  // 0 or 1: one product
-    long long bsa, bsb, bsc;
-};
-
 // GATHER (sampled amplitudes): row i of A and C is row rows[i] of the arrays
 // (negative: none), and B is shifted by digit * bdig, one digit per TM rows
 // (negative: no row; >= ndig: the product is zero).
@@ -214,41 +193,16 @@ struct GemmGather {
     int ndig;
 };
 
-__device__ __forceinline__ void copy8_async(uint32_t dst, const void* src, uint32_t bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes)
-                 : "memory");
-}
-
 struct GemmLaunch {
     GemmArgs p[2];
     int two;                    // blockIdx.z selects p[0] or p[1], else the batch
     GemmGather ga;
 };
 
-// acc += a b, or a conj(b).
-template <bool CONJ>
-__device__ __forceinline__ void cfma_op(cf& acc, cf a, cf b) {
-    if (CONJ) {
-        acc.x = fmaf(a.x, b.x, fmaf(a.y, b.y, acc.x));
-        acc.y = fmaf(a.y, b.x, fmaf(-a.x, b.y, acc.y));
-    } else {
-        cfma(acc, a, b);
-    }
-}
-
-// CONJ: the second factor is conjugated; a conjugated first factor is the
-// conjugate of the product with the second one's conjugation flipped.
 template <int TM, int TN, int KS, bool CONJ, bool GATHER>
 __global__ void __launch_bounds__(256, 2) cgemm_kernel(const __grid_constant__ GemmLaunch gl) {
-    constexpr int KC = KS > 1 ? 16 : 8;                       // K of a chunk
-    constexpr int ST = 4;                                     // chunks in shared memory
-    constexpr int GT = 256 / KS;                              // threads of a group
-    constexpr int XN = TN / 4, XM = TM / 4;
-    constexpr int NA = TM * KC / 256, NB = TN * KC / 256;     // loads a thread and chunk
-    static_assert(XN * XM == GT, "4 x 4 outputs a thread");
-    constexpr int BUF = KC * (TM + 1 + TN + 1);
-    __shared__ __align__(16) cf sm[ST * BUF];
-    static_assert((KS - 1) * TM * TN <= ST * BUF, "the groups' sums fit");
+    using Tile = GemmTile<TM, TN, KS>;
+    __shared__ __align__(16) cf sm[Tile::ST * Tile::BUF];
     GemmArgs g = gl.p[gl.two && blockIdx.z ? 1 : 0];
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
     if (m0 >= g.M || n0 >= g.N) return;
@@ -263,132 +217,17 @@ __global__ void __launch_bounds__(256, 2) cgemm_kernel(const __grid_constant__ G
         if (x >= gl.ga.ndig) g.K = 0;
         else g.B += x * gl.ga.bdig;
     }
-    const int tid = threadIdx.x, grp = tid / GT, t = tid % GT, tx = t % XN, ty = t / XN;
-    // this thread's elements of a chunk, along the unit stride of each operand:
-    // source (of chunk 0), K index (beyond K for an absent row or column)
-    const bool a_kfast = g.sak == 1, b_nfast = g.sbn == 1;
-    int ak[NA], bk[NB];
-    uint32_t ad[NA], bd[NB];
-    const cf* ap[NA];
-    const cf* bp[NB];
-    const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
-#pragma unroll
-    for (int q = 0; q < NA; ++q) {
-        const int e = tid + 256 * q;
-        const int k = a_kfast ? e % KC : e / TM, r = a_kfast ? e / KC : e % TM;
-        int row = m0 + r;
-        bool in = row < g.M;
-        if (GATHER && in) {
-            row = gl.ga.rows[row];
-            in = row >= 0;
-        }
-        ak[q] = in ? k : INT_MAX;
-        ad[q] = base + (k * (TM + 1) + r) * (uint32_t)sizeof(cf);
-        ap[q] = in ? g.A + row * g.sam + k * g.sak : g.A;
-    }
-#pragma unroll
-    for (int q = 0; q < NB; ++q) {
-        const int e = tid + 256 * q;
-        const int k = b_nfast ? e / TN : e % KC, c = b_nfast ? e % TN : e / KC;
-        const int col = n0 + c;
-        bk[q] = col < g.N ? k : INT_MAX;
-        bd[q] = base + (KC * (TM + 1) + k * (TN + 1) + c) * (uint32_t)sizeof(cf);
-        bp[q] = col < g.N ? g.B + k * g.sbk + col * g.sbn : g.B;
-    }
-    const long long da = KC * g.sak, db = KC * g.sbk;
-    const int chunks = (g.K + KC - 1) / KC;
-    // chunk c into buffer c mod ST by 8-byte asynchronous copies (zeros past K)
-    const auto fetch = [&](int c) {
-        if (c < chunks) {
-            const int left = g.K - c * KC;
-            const uint32_t off = (uint32_t)((c & (ST - 1)) * BUF) * (uint32_t)sizeof(cf);
-#pragma unroll
-            for (int q = 0; q < NA; ++q) {
-                const bool in = ak[q] < left;
-                copy8_async(ad[q] + off, in ? ap[q] : g.A, in ? 8u : 0u);
-                ap[q] += da;
-            }
-#pragma unroll
-            for (int q = 0; q < NB; ++q) {
-                const bool in = bk[q] < left;
-                copy8_async(bd[q] + off, in ? bp[q] : g.B, in ? 8u : 0u);
-                bp[q] += db;
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    cf acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = cmake(0.f, 0.f);
-#pragma unroll
-    for (int c = 0; c < ST - 1; ++c) fetch(c);
-    for (int c = 0; c < chunks; ++c) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
-        __syncthreads();
-        fetch(c + ST - 1);
-        const cf* As = sm + (c & (ST - 1)) * BUF;
-        const cf* Bs = As + KC * (TM + 1);
-#pragma unroll
-        for (int kk = 0; kk < KC / KS; ++kk) {
-            const int k = kk * KS + grp;
-            cf av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = As[k * (TM + 1) + ty + XM * i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bv[j] = Bs[k * (TN + 1) + tx + XN * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) cfma_op<CONJ>(acc[i][j], av[i], bv[j]);
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    if (KS > 1) {
-        if (grp > 0) {
-            cf* dst = sm + (size_t)(grp - 1) * TM * TN;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dst[(4 * i + j) * GT + t] = acc[i][j];
-        }
-        __syncthreads();
-        if (grp > 0) return;
-#pragma unroll
-        for (int q = 0; q < KS - 1; ++q)
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[i][j] = cadd(acc[i][j], sm[(size_t)q * TM * TN + (4 * i + j) * GT + t]);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int row = m0 + ty + XM * i;
-        if (row >= g.M) continue;
-        if (GATHER) {
-            row = gl.ga.rows[row];
-            if (row < 0) continue;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int col = n0 + tx + XN * j;
-            if (col < g.N)
-                g.C[row * g.scm + col * g.scn] = g.conjA ? cconj(acc[i][j]) : acc[i][j];
-        }
-    }
+    Tile::template run<CONJ, GATHER>(g, m0, n0, gl.ga.rows, sm, [&](int row, int col, cf v) {
+        g.C[row * g.scm + col * g.scn] = v;
+    });
 }
 
 // 64 x 64 tiles once they give every SM a CTA, else 32 x 32 (four times the tiles,
 // the K loop split over four groups of threads).  Measured with each: 64 steps
 // of two 256 x 512 x 256 products (64 large tiles), 2.64 ms small against 5.00
 // large; 64 products of 4096 x 256 x 256 (256 large tiles), 3.13 against 3.05.
-constexpr int kGemmSms = 152;
-
 bool small_tiles(long long m, long long n, long long count) {
-    return ((m + 63) / 64) * ((n + 63) / 64) * count < kGemmSms;
+    return ((m + 63) / 64) * ((n + 63) / 64) * count < kSms;
 }
 
 int cgemm_launch(const GemmLaunch& gl, int m, int n, int z, cudaStream_t s) {

@@ -90,7 +90,8 @@ struct Slot {
     float scale[GS_W];                       // the columns' scales at the end, less 1
     alignas(8) unsigned mask[GS_W];          // pairs that rotate in a step
     int col[GS_W];                           // physical columns
-    int job, I, J, full, L, vrows;        // the visit (job < 0: no more)
+    int job, I, J, full, L, vrows;
+    float tol2;        // the visit (job < 0: no more)
     int time, changedI, changedJ;            // its time, when its blocks last changed
     int* qst;                                // its quiet stamp
     int work;
@@ -544,7 +545,8 @@ struct Turn {
 // the next item is claimed and its job looked up while the present one is on
 // its way.
 template <int LW, int S, int NG>
-__device__ __forceinline__ void loader(const TwoQGeom& g, const SweepSync& sync, int tbase, cf* Xs,
+__device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const SweepSync& sync,
+                                       int tbase, cf* Xs,
                                        Slot<NG>* slots, int lane) {
     constexpr int XST = LW + 2;
     const int4 head = __ldcg(g.gact);         // jobs left, their rounds and pairs
@@ -664,6 +666,7 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, const SweepSync& sync,
                 sl.full = r == 0 ? 1 : 0;
                 sl.L = L;
                 sl.vrows = vrows;
+                sl.tol2 = tol2 > 0.f ? tol2 : default_tol2(slot_rows(L));
                 sl.time = tbase + r + 1;
                 sl.changedI = cI;
                 sl.changedJ = cJ;
@@ -712,8 +715,8 @@ __device__ __forceinline__ void gram_role(const SweepSync& sync, const cf* Xs, S
 }
 
 template <int LW, int S, int NG>
-__device__ __forceinline__ void solver_role(const TwoQGeom& g, float tol2, const SweepSync& sync,
-                                            Slot<NG>& sl, int lane) {
+__device__ __forceinline__ void solver_role(const TwoQGeom& g, const SweepSync& sync, Slot<NG>& sl,
+                                            int lane) {
     bool expired = false;
     for (unsigned par = 0u;; par ^= 1u) {
         slot_wait(&sl.b_info, par, expired);
@@ -727,6 +730,7 @@ __device__ __forceinline__ void solver_role(const TwoQGeom& g, float tol2, const
         }
         const int I = sl.I, J = sl.J;
         const bool full = sl.full != 0;
+        const float tol2 = sl.tol2;
         cf* GI = g.gblk + ((size_t)j * (g.cslot / GS_BC) + I) * GS_NP;
         cf* GJ = g.gblk + ((size_t)j * (g.cslot / GS_BC) + J) * GS_NP;
         if (!full) {
@@ -899,8 +903,8 @@ gram_sweep_kernel(TwoQGeom g, float tol2, SweepSync sync, int tbase) {
     }
     __syncthreads();
     const int role = (int)(blockDim.x >> 5) - 1 - warp;          // apply warps first
-    if (role == 0) loader<LW, S, NG>(g, sync, tbase, Xs, slots, lane);
-    else if (role <= S) solver_role<LW, S, NG>(g, tol2, sync, slots[role - 1], lane);
+    if (role == 0) loader<LW, S, NG>(g, tol2, sync, tbase, Xs, slots, lane);
+    else if (role <= S) solver_role<LW, S, NG>(g, sync, slots[role - 1], lane);
     else if (role <= S + NG) gram_role<LW, S, NG>(sync, Xs, slots, role - 1 - S, lane);
     else apply_role<LW, S, NG, NA>(g, sync, Xs, slots, role - 1 - S - NG, lane);
 }
@@ -1015,13 +1019,15 @@ int gram_begin_launch(const mps_2q_job* jobs, int njobs, const TwoQGeom& g, cons
 int gram_sweep_launch(int njobs, int rounds, int pairs, const TwoQGeom& g,
                       float tol2, const SweepSync& sync, int tbase, cudaStream_t s) {
     if (!g.gblk || !g.gstate || !g.gact || !g.qstamp) return fail(MPS_ERR_ARG, "gram sweeps: no block products");
+    // (three Gram warps everywhere: a product's partial sums, and so its rounding,
+    // do not depend on the slot a job happens to share with others)
     switch (g.lslot) {
-        case 64: return launch<64, 4, 2, 5>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 64: return launch<64, 4, 3, 4>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
         case 128: return launch<128, 4, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
         case 256: return launch<256, 4, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
         case 512: return launch<512, 3, 3, 9>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
-        case 576: return launch<576, 2, 4, 9>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
-        case 1024: return launch<1024, 1, 4, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 576: return launch<576, 2, 3, 10>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 1024: return launch<1024, 1, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
         default: return fail(MPS_ERR_ARG, "gram sweeps: unsupported slot size");
     }
 }

@@ -35,11 +35,12 @@
 // Column norms are recomputed from the data at every visit, so they do not
 // drift.
 //
-// V.  A job that is tall (m >= n) and left-canonical -- the default of
-// apply_two_qudit_gate -- needs only U = X_k / S: one Newton-Schulz step makes
-// U an isometry to rounding, and its right site S V^H equals U^H theta, one
-// GEMM against a copy of theta, so such jobs never accumulate V.  Other jobs accumulate the 2BC x 2BC rotation of each visit in
-// shared memory and apply V <- V Q.
+// V.  Where X's left factor is the isometric site (every square theta; a tall one
+// left-canonical, the default of apply_two_qudit_gate; a somewhat wide one
+// right-canonical) only U = X_k / S is needed: one Newton-Schulz step makes U an
+// isometry to rounding, and the other site is one product of U^H with a copy of
+// X, so such jobs never accumulate V (job_tracks_v).  Other jobs accumulate the
+// rotations of each visit in V.
 //
 // Afterwards sigma_c = |X_c|, sorted descending (ties by column index); the
 // first k are kept.  Where the isometric factor would divide by an exact-zero
@@ -50,6 +51,7 @@
 #include <mutex>
 #include <string>
 
+#include "gemm.cuh"
 #include "rot.cuh"
 #include "twoq.cuh"
 
@@ -59,7 +61,7 @@ namespace {
 
 struct JobShape {
     int m, n, L, C, nb;
-    bool tall, track_v;
+    bool track_v;
 };
 
 template <int BC>
@@ -69,7 +71,6 @@ __device__ __forceinline__ JobShape job_shape(const mps_2q_job* jobs, int j, int
     s.n = jobs[j].chi_r * d;
     s.L = max(s.m, s.n);
     s.C = min(s.m, s.n);
-    s.tall = s.m >= s.n;
     s.track_v = job_tracks_v(s.m, s.n, jobs[j].keep_left_canonical);
     int nb = (s.C + BC - 1) / BC;
     if (nb < 2) nb = 2;
@@ -860,8 +861,8 @@ sort_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int npow2) {
         double tot = 0.0;
         for (int w = 0; w < SORT_T / 32; ++w) tot += s_red[w];
         if (job.discarded) *job.discarded = tot;
-        const bool tall = m >= n;
-        const bool divides = tall ? (job.keep_left_canonical != 0) : (job.keep_left_canonical == 0);
+        // the isometric site is X divided by the singular values
+        const bool divides = job.keep_left_canonical ? m >= n : m <= n;
         int need = 0;
         if (divides)
             for (int i = 0; i < k; ++i) need += (key[i] <= thr) ? 1 : 0;
@@ -878,8 +879,9 @@ sort_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int npow2) {
 }
 
 // a_out (m x k, row-major): a_out[row*k + i] = scale_i * src[perm_i * ld + row]
-//   tall: src = X (U S columns), scale = 1/s (left-canonical) or 1
-//   wide: src = V,               scale = 1 (left-canonical) or s
+//   X = theta:    src = X (U S columns), scale = 1/s (left-canonical) or 1
+//   X = theta^H:  src = V, scale = 1 (left-canonical) or s
+// (X = theta^T: the left site is one of launch_post's products.)
 __global__ void regauge_a_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
     __shared__ cf tile[32][33];
     const int j = blockIdx.z;
@@ -888,8 +890,9 @@ __global__ void regauge_a_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g
     const int k = job.k;
     const int i0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     if (i0 >= k || r0 >= m) return;
-    const bool tall = m >= n;
+    const bool tall = job_tall(m, n, job.keep_left_canonical);
     const bool lc = job.keep_left_canonical != 0;
+    if (!tall && !job_tracks_v(m, n, job.keep_left_canonical)) return;
     const cf* src;
     int ld;
     if (tall) { src = g.X + (size_t)j * g.lslot * g.cslot; ld = g.lslot; }
@@ -918,155 +921,119 @@ __global__ void regauge_a_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g
     }
 }
 
-// b_out (k x n, row-major) for jobs that track V:
-//   tall (right-canonical): b_out[i, :] = conj(V[:, perm_i])
-//   wide: b_out[i, :] = scale_i * conj(X[:, perm_i]), scale = 1 (lc) or 1/s
+// b_out (k x n, row-major):
+//   X = theta, right-canonical:  b_out[i, :] = conj(V[:, perm_i])
+//   X = theta^H:                 b_out[i, :] = scale * conj(X[:, perm_i]), 1 or 1/s
+//   X = theta^T:                 b_out[i, :] = X[:, perm_i] / s
+// (X = theta, left-canonical: the right site is one of launch_post's products.)
 __global__ void regauge_b_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
     const int j = blockIdx.z;
     const mps_2q_job job = jobs[j];
     const int m = job.chi_l * g.d, n = job.chi_r * g.d;
     const int i = blockIdx.y;
     if (i >= job.k) return;
-    if (!job_tracks_v(m, n, job.keep_left_canonical)) return;
-    const bool tall = m >= n;
+    const bool tall = job_tall(m, n, job.keep_left_canonical);
     const bool lc = job.keep_left_canonical != 0;
+    if (tall && lc) return;
     const cf* src;
     int ld;
     if (tall) { src = g.V + (size_t)j * g.cslot * g.cslot; ld = g.cslot; }
     else { src = g.X + (size_t)j * g.lslot * g.cslot; ld = g.lslot; }
     const float* sig = g.sig + (size_t)j * g.cslot;
     const float thr = kZeroSigma * fmaxf(sig[0], 1.f);
-    const float s = sig[i];
-    float sc;
-    if (tall) sc = 1.f;
-    else sc = lc ? 1.f : (s > thr ? 1.f / s : 0.f);
+    const bool transposed = !tall && !job_tracks_v(m, n, job.keep_left_canonical);
+    const float s = sig[i], sc = !tall && !lc ? (s > thr ? 1.f / s : 0.f) : 1.f;
     const cf* col = src + (size_t)g.perm[(size_t)j * g.cslot + i] * ld;
     cf* out = reinterpret_cast<cf*>(job.b_out) + (size_t)i * n;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-        out[c] = cscale(cconj(col[c]), sc);
+        out[c] = cscale(transposed ? col[c] : cconj(col[c]), sc);
 }
 
-// Post-processing GEMMs for tall left-canonical jobs (the V-free path), all
-// 64x64 output tiles, K in chunks of 16, 256 threads x 4x4 outputs:
-//   POST_GRAM : G = U^H U          (k x k, into the job's V slot), U = a_out
-//   POST_APPLY: U' = U (3I - G)/2  (m x k, into the job's X slot): one
+// Products that finish the V-free jobs.  With Z = theta (left-canonical) or
+// theta^T (right-canonical), p x q, and U its left factor as the regauge left
+// it in the isometric site (a_out, p x k row-major, or b_out, its transpose):
+//   POST_GRAM : G = U^H U            (k x k, into the job's V slot)
+//   POST_APPLY: U' = U (3I - G)/2    (laid out like U, into the job's X slot): one
 //               Newton-Schulz step, which squares U's distance from an
 //               isometry (the Jacobi tolerance) so U U^H is a projector to
 //               rounding, as LAPACK's U would give
-//   POST_UH   : S V^H = U'^H theta (k x n, into b_out), theta = the T copy
-//   POST_COPY : a_out = U'
+//   POST_UH   : S W^H = U'^H Z       (k x q, into the other site), Z = the T copy
+// and post_copy_kernel puts U' in the isometric site.  64 x 64 tiles of gemm.cuh
+// for every size: 32 x 32 ones measured no better for small calls either (layers
+// of 48 sites chi=128, 5.87 against 6.08 ms; 64 sites chi=256, 20.8 against 21.2),
+// and one tile for all keeps a job's rounding independent of its call.
 enum PostMode { POST_GRAM = 0, POST_APPLY = 1, POST_UH = 2 };
 
 template <int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 post_gemm_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
-    __shared__ cf As[16][64];
-    __shared__ cf Bs[16][64];
+    constexpr int TM = 64, TN = 64;
+    using Tile = GemmTile<TM, TN, 1>;
+    __shared__ __align__(16) cf sm[Tile::ST * Tile::BUF];
     const int j = blockIdx.z;
     const mps_2q_job job = jobs[j];
     const int m = job.chi_l * g.d, n = job.chi_r * g.d, k = job.k;
     if (job_tracks_v(m, n, job.keep_left_canonical)) return;
-    int M, N, K;
-    if (MODE == POST_GRAM) { M = k; N = k; K = m; }
-    else if (MODE == POST_APPLY) { M = m; N = k; K = k; }
-    else { M = k; N = n; K = m; }
-    const int i0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-    if (i0 >= M || c0 >= N) return;
-    const cf* U = reinterpret_cast<const cf*>(job.a_out);          // m x k row-major
-    cf* Gm = g.V + (size_t)j * g.cslot * g.cslot;                   // k x k row-major
-    cf* Up = g.X + (size_t)j * g.lslot * g.cslot;                   // m x k row-major
-    const cf* T = g.T + (size_t)j * g.lslot * g.cslot;              // theta, column-major
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    cf acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = cmake(0.f, 0.f);
-    for (int l0 = 0; l0 < K; l0 += 16) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int idx = tid + q * 256;
-            int ti, kk;
-            if (MODE == POST_APPLY) { kk = idx & 15; ti = idx >> 4; }   // U rows: l contiguous
-            else { ti = idx & 63; kk = idx >> 6; }                     // U^H: i contiguous
-            const int i = i0 + ti, l = l0 + kk;
-            cf v = cmake(0.f, 0.f);
-            if (i < M && l < K) {
-                if (MODE == POST_GRAM) v = cconj(U[(size_t)l * k + i]);
-                else if (MODE == POST_APPLY) v = U[(size_t)i * k + l];
-                else v = cconj(Up[(size_t)l * k + i]);
-            }
-            As[kk][ti] = v;
+    const bool lc = job.keep_left_canonical != 0;
+    const int p = lc ? m : n, q = lc ? n : m;
+    const cf* U = reinterpret_cast<const cf*>(lc ? job.a_out : job.b_out);
+    cf* other = reinterpret_cast<cf*>(lc ? job.b_out : job.a_out);
+    cf* Gm = g.V + (size_t)j * g.cslot * g.cslot;
+    cf* Up = g.X + (size_t)j * g.lslot * g.cslot;
+    const cf* T = g.T + (size_t)j * g.lslot * g.cslot;              // Z, column-major
+    const long long ul = lc ? k : 1, ui = lc ? 1 : p;               // strides of U and U'
+    GemmArgs a{};
+    if (MODE == POST_GRAM) a = GemmArgs{k, k, p, U, ui, ul, 1, U, ul, ui, 0, Gm, k, 1};
+    // (right-canonical: rows and columns swapped, so that consecutive outputs
+    // stay consecutive in memory)
+    else if (MODE == POST_APPLY)
+        a = lc ? GemmArgs{p, k, k, U, ul, ui, 0, Gm, k, 1, 0, Up, ul, ui}
+               : GemmArgs{k, p, k, Gm, 1, k, 0, U, ui, ul, 0, Up, ui, ul};
+    else
+        a = lc ? GemmArgs{k, q, p, Up, ui, ul, 1, T, 1, g.lslot, 0, other, q, 1}
+               : GemmArgs{q, k, p, T, g.lslot, 1, 0, Up, ul, ui, 1, other, k, 1};
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+    if (m0 >= a.M || n0 >= a.N) return;
+    Tile::template run<MODE != POST_APPLY, false>(a, m0, n0, nullptr, sm, [&](int r, int c, cf v) {
+        if (MODE == POST_APPLY) {
+            const cf u = U[r * a.scm + c * a.scn];
+            v = cmake(1.5f * u.x - 0.5f * v.x, 1.5f * u.y - 0.5f * v.y);
         }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int idx = tid + q * 256;
-            int tc, kk;
-            if (MODE == POST_UH) { kk = idx & 15; tc = idx >> 4; }      // theta column-major
-            else { tc = idx & 63; kk = idx >> 6; }
-            const int c = c0 + tc, l = l0 + kk;
-            cf v = cmake(0.f, 0.f);
-            if (c < N && l < K) {
-                if (MODE == POST_GRAM) v = U[(size_t)l * k + c];
-                else if (MODE == POST_APPLY) {
-                    const cf gl = Gm[(size_t)l * k + c];
-                    v = cmake((l == c ? 1.5f : 0.f) - 0.5f * gl.x, -0.5f * gl.y);
-                } else v = T[(size_t)c * g.lslot + l];
-            }
-            Bs[kk][tc] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            cf av[4], bv[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) av[a] = As[kk][ty + 16 * a];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) bv[b] = Bs[kk][tx + 16 * b];
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) cfma(acc[a][b], av[a], bv[b]);
-        }
-        __syncthreads();
-    }
-    cf* out;
-    size_t ld;
-    if (MODE == POST_GRAM) { out = Gm; ld = (size_t)k; }
-    else if (MODE == POST_APPLY) { out = Up; ld = (size_t)k; }
-    else { out = reinterpret_cast<cf*>(job.b_out); ld = (size_t)n; }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int i = i0 + ty + 16 * a, c = c0 + tx + 16 * b;
-            if (i < M && c < N) out[(size_t)i * ld + c] = acc[a][b];
-        }
+        a.C[r * a.scm + c * a.scn] = v;
+    });
 }
 
-// a_out = U' (the X slot) for tall left-canonical jobs.
+// The isometric site = U' (the X slot) for the V-free jobs.
 __global__ void post_copy_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
     const int j = blockIdx.y;
     const mps_2q_job job = jobs[j];
     const int m = job.chi_l * g.d, n = job.chi_r * g.d;
     if (job_tracks_v(m, n, job.keep_left_canonical)) return;
-    const size_t total = (size_t)m * job.k;
+    const bool lc = job.keep_left_canonical != 0;
+    const size_t total = (size_t)(lc ? m : n) * job.k;
     const cf* src = g.X + (size_t)j * g.lslot * g.cslot;
-    cf* dst = reinterpret_cast<cf*>(job.a_out);
+    cf* dst = reinterpret_cast<cf*>(lc ? job.a_out : job.b_out);
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
          e += (size_t)gridDim.x * blockDim.x)
         dst[e] = src[e];
 }
 
+template <int MODE>
+int launch_post_gemm(const mps_2q_job* jobs, int njobs, int rows, int cols, const TwoQGeom& g,
+                     cudaStream_t s) {
+    const dim3 grid((cols + 63) / 64, (rows + 63) / 64, njobs);
+    post_gemm_kernel<MODE><<<grid, 256, 0, s>>>(jobs, g);
+    MPS_LAUNCH_CHECK("post_gemm_kernel");
+    return MPS_OK;
+}
+
 int launch_post(const mps_2q_job* jobs, int njobs, int max_m, int max_n, int kmax,
                 const TwoQGeom& g, cudaStream_t s) {
-    post_gemm_kernel<POST_GRAM><<<dim3((kmax + 63) / 64, (kmax + 63) / 64, njobs), 256, 0, s>>>(jobs, g);
-    MPS_LAUNCH_CHECK("post_gemm_kernel<gram>");
-    post_gemm_kernel<POST_APPLY><<<dim3((kmax + 63) / 64, (max_m + 63) / 64, njobs), 256, 0, s>>>(jobs, g);
-    MPS_LAUNCH_CHECK("post_gemm_kernel<apply>");
-    post_gemm_kernel<POST_UH><<<dim3((max_n + 63) / 64, (kmax + 63) / 64, njobs), 256, 0, s>>>(jobs, g);
-    MPS_LAUNCH_CHECK("post_gemm_kernel<uh>");
-    const size_t total = (size_t)max_m * kmax;
+    const int side = max(max_m, max_n);       // U' and the other factor, in either form
+    if (int rc = launch_post_gemm<POST_GRAM>(jobs, njobs, kmax, kmax, g, s)) return rc;
+    if (int rc = launch_post_gemm<POST_APPLY>(jobs, njobs, side, side, g, s)) return rc;
+    if (int rc = launch_post_gemm<POST_UH>(jobs, njobs, side, side, g, s)) return rc;
+    const size_t total = (size_t)side * kmax;
     int blocks = (int)((total + 255) / 256 < 1024 ? (total + 255) / 256 : 1024);
     post_copy_kernel<<<dim3(blocks > 0 ? blocks : 1, njobs), 256, 0, s>>>(jobs, g);
     MPS_LAUNCH_CHECK("post_copy_kernel");
@@ -1074,8 +1041,9 @@ int launch_post(const mps_2q_job* jobs, int njobs, int max_m, int max_n, int kma
 }
 
 // Orthonormal completion of the isometric factor where sigma is an exact
-// zero.  Vectors u_i (i < k): tall -> columns of a_out (R = m, element
-// stride k); wide -> rows of b_out (R = n, element stride 1).  The columns
+// zero (where the isometric site divides by S).  Vectors u_i (i < k): left-canonical -> columns of a_out
+// (R = m, element stride k); right-canonical -> rows of b_out (R = n, element
+// stride 1).  The columns
 // needing completion are a suffix of the kept set (sigma sorted).
 constexpr int COMP_T = 256;
 
@@ -1087,7 +1055,7 @@ complete_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
     if (need == 0) return;
     const mps_2q_job job = jobs[j];
     const int m = job.chi_l * g.d, n = job.chi_r * g.d;
-    const bool tall = m >= n;
+    const bool tall = job.keep_left_canonical != 0;
     const int k = job.k;
     const int R = tall ? m : n;
     cf* base = reinterpret_cast<cf*>(tall ? job.a_out : job.b_out);
@@ -1380,15 +1348,6 @@ struct Layout {
     int nbmax, qstride;
 };
 
-// Column length of a slot: the ring kernel reads exactly 32*ROWS rows, so
-// the slot is padded up to the ROWS step pick_visit chooses for it.
-int slot_rows(int L) {
-    const int steps[] = {64, 128, 256, 512, 576, 1024, 1792};
-    for (int r : steps)
-        if (L <= r) return r;
-    return (int)align_up((size_t)L, 32);
-}
-
 Layout make_layout(int njobs, int max_m, int max_n, bool pieces = false, bool gram = true) {
     Layout lo;
     const int L = max(max_m, max_n), C = min(max_m, max_n);
@@ -1532,14 +1491,9 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
         if (params->max_sweeps > 0) max_sweeps = params->max_sweeps;
         tol = params->tol;
     }
-    // The computed x_p^H x_q carries a rounding error of a few 2^-24
-    // sum_r |x_r||q_r|, growing slowly with the length L; the default
-    // threshold 2^-24 max(8, sqrt(L)) stays above that noise (no sweep keeps
-    // rotating noise) while the kept subspace -- whose error is about
-    // tol s_k / gap at the truncation cut -- stays close to what a
-    // backward-stable complex64 SVD gives.
-    if (!(tol > 0.f)) tol = 5.9604645e-8f * fmaxf(8.f, sqrtf((float)lo.lslot));
-    const float tol2 = tol * tol;     // the kernels compare squared cosines
+    // the kernels compare squared cosines (asked: the caller's tolerance, if any)
+    const float asked = tol > 0.f ? tol * tol : 0.f;
+    const float tol2 = asked > 0.f ? asked : default_tol2(lo.lslot);
     const bool mixed = params && params->precision == MPS_PRECISION_MIXED;
     if (params && params->precision != MPS_PRECISION_PLAIN && !mixed)
         return fail(MPS_ERR_ARG, "mps_apply_2q_batch: unknown precision");
@@ -1631,7 +1585,7 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
                                                                        sweeps * tbase_stride);
                     MPS_LAUNCH_CHECK("presort_kernel");
                 }
-                rc = gram_sweep_launch(njobs, rounds, pairs, g, tol2, sync, sweeps * tbase_stride, s);
+                rc = gram_sweep_launch(njobs, rounds, pairs, g, asked, sync, sweeps * tbase_stride, s);
                 if (rc) return rc;
             }
             if (sweeps == 1) continue;
@@ -1688,7 +1642,7 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
             // the SIMT jobs (all of them in the plain form): one persistent
             // launch runs every round of the sweep
             if (simt_left) {
-                rc = gram ? gram_sweep_launch(njobs, rounds, pairs, g, tol2, sync,
+                rc = gram ? gram_sweep_launch(njobs, rounds, pairs, g, asked, sync,
                                               sweeps * tbase_stride, s)
                           : launch_sweep<8, 56>(jobs, njobs, rounds, pairs, g, tol2, lw, sync,
                                                 sweeps * tbase_stride, s);
@@ -1884,8 +1838,7 @@ extern "C" int mps_apply_2q_batch_noalloc(void* stream, const mps_2q_job* jobs, 
         if (params->max_sweeps > 0) max_sweeps = params->max_sweeps;
         tol = params->tol;
     }
-    if (!(tol > 0.f)) tol = 5.9604645e-8f * fmaxf(8.f, sqrtf((float)lo.lslot));
-    const float tol2 = tol * tol;     // the kernels compare squared cosines
+    const float tol2 = tol > 0.f ? tol * tol : default_tol2(lo.lslot);
     const int lw = lo.lslot;
     int bc = 16;
     visit_fn visit = pick_visit(lw, &bc);

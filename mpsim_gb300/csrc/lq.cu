@@ -1,8 +1,8 @@
 // lq.cu -- LQ preconditioning of the Jacobi SVD (sm_103a).
 //
-// For a job whose left factor is read off the final Jacobi columns (theta
-// tall or square, keep_left_canonical: X = theta, L x C, column-major in the
-// X slot), X is replaced by its L factor before the sweeps:
+// For a job whose isometric factor is read off the final Jacobi columns (X =
+// theta or theta^T, L x C with L >= C, column-major in the X slot: job_tracks_v),
+// X is replaced by its L factor before the sweeps:
 //
 //     X = L Q,  Q (C x C) unitary,  L (L x C) lower trapezoidal.
 //
@@ -52,8 +52,8 @@ static_assert(LQ_MIN_C * LQ_MIN_C >= LQ_B * (LQ_MIN_C + LQ_B), "V slot too small
 __device__ __forceinline__ bool lq_job(const mps_2q_job& job, int d, int& L, int& C) {
     const int m = job.chi_l * d, n = job.chi_r * d;
     if (job_tracks_v(m, n, job.keep_left_canonical)) return false;
-    L = m;
-    C = n;
+    L = max(m, n);
+    C = min(m, n);
     return C >= LQ_MIN_C && C <= LQ_MAX_C;
 }
 
@@ -360,7 +360,7 @@ int lq_precondition(const mps_2q_job* jobs, int njobs, int max_m, int max_n, con
     for (int k0 = 0; k0 < cmax; k0 += LQ_B) {
         lq_panel_kernel<<<njobs, LQ_T, smem, s>>>(jobs, g, k0);
         MPS_LAUNCH_CHECK("lq_panel_kernel");
-        const int rows = max_m - k0;     // covers every job's rows below its panel
+        const int rows = max(max_m, max_n) - k0;   // covers every job's rows below its panel
         if (rows > 0) {
             lq_trail_kernel<<<dim3((rows + LQ_TR - 1) / LQ_TR, njobs), 256, 0, s>>>(jobs, g, k0);
             MPS_LAUNCH_CHECK("lq_trail_kernel");

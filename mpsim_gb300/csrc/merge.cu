@@ -8,7 +8,7 @@
 // columns are (b, r) for TR = 64/d values of r and all b -- exactly the
 // entries the gate needs for the same theta tile -- then mixes the tile with
 // the gate in shared memory and writes theta straight into the Jacobi working
-// matrix X (column-major; conjugate-transposed for wide theta).
+// matrix X (column-major; transposed or conjugate-transposed as job_tall says).
 //
 // A job flagged MPS_JOB_THETA_GIVEN carries theta itself: a points to the
 // (chi_l*d) x (d*chi_r) matrix, row-major, and the same CTAs copy their tile
@@ -34,7 +34,7 @@ merge_gate_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
     const int l0 = blockIdx.y * TL, r0 = blockIdx.x * TR;
     if (l0 >= chil || r0 >= chir) return;
     const int m = chil * d, n = d * chir;
-    const bool tall = m >= n;
+    const bool tall = job_tall(m, n, job.keep_left_canonical);
     const bool given = (job.flags & MPS_JOB_THETA_GIVEN) != 0;   // block-uniform
     if (g.tc_mode && merge_on_tensor_cores(job, d)) return;       // merge_tc_kernel's job
 
@@ -122,8 +122,11 @@ merge_gate_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
         if (tall) {
             X[(size_t)tcol * g.lslot + trow] = th;
             if (!track_v) T[(size_t)tcol * g.lslot + trow] = th;
-        } else {
+        } else if (track_v) {
             X[(size_t)trow * g.lslot + tcol] = cconj(th);
+        } else {
+            X[(size_t)trow * g.lslot + tcol] = th;
+            T[(size_t)trow * g.lslot + tcol] = th;
         }
     }
 }

@@ -1,11 +1,12 @@
 // Workspace geometry shared by the two-qudit kernels (merge, Jacobi SVD,
 // sort, regauge).  One slot per job; every job's slot has the same shape.
 //
-// For a job with theta of m x n (m = chi_l*d, n = d*chi_r):
-//   tall (m >= n): the Jacobi matrix X is theta itself, column-major,
-//                  C = n columns of length L = m.  X V = U S.
-//   wide (m <  n): X is theta^H (conjugate transpose), C = m columns of
-//                  length L = n.  theta = V S (X/S)^H.
+// For a job with theta of m x n (m = chi_l*d, n = d*chi_r), C = min(m, n) columns
+// of length L = max(m, n) (see job_tall and job_tracks_v):
+//   X = theta    X V = U S
+//   X = theta^H  (wide, V tracked)   theta = V S (X/S)^H
+//   X = theta^T  (wide or square, right-canonical, V not tracked)
+//                X V = U S, theta = conj(V) S U^T
 // X: lslot x cslot complex64, column-major (column c at X + c*lslot).
 // V: cslot x cslot complex64, column-major, starts as the identity.
 #pragma once
@@ -73,17 +74,31 @@ struct SweepSync {
     int stall_test;
 };
 
-// A job tracks the right rotations V unless it is tall (m >= n) and left-
-// canonical: then U = X/S is all the Jacobi iteration must produce, and the
-// right site S V^H = U^H theta comes from one GEMM against a copy of theta.
+// A job's X and whether it tracks the right rotations V.  The factor that must
+// come out isometric is the left one (keep_left_canonical) or the right one;
+// let Z = theta in the first case and theta^T in the second, so that it is
+// the left factor of Z.  Where Z has at least as many rows as columns (every
+// square theta, in both forms), X = Z, U = X/S of the final columns is all the
+// Jacobi iteration must produce, and the other factor S W^H = U^H Z is one
+// product with a copy of Z.  The others (a wide theta left-canonical, a tall one
+// right-canonical) work on the other side, X = Z^H, and accumulate V.  So does a
+// right-canonical theta at least twice as wide as tall: the few rows of V cost
+// less than finishing long columns (a 14-qubit from_wavefunction, whose blocks
+// are such, takes 14.5 ms so and 16.4 otherwise).
 __host__ __device__ __forceinline__ bool job_tracks_v(int m, int n, int keep_left_canonical) {
-    return !(m >= n && keep_left_canonical != 0);
+    return keep_left_canonical != 0 ? m < n : (m > n || n >= 2 * m);
+}
+
+// Whether X holds theta itself (its columns); else theta's conjugate transpose
+// (jobs that track V) or transpose (the others).
+__host__ __device__ __forceinline__ bool job_tall(int m, int n, int keep_left_canonical) {
+    return keep_left_canonical != 0 ? m >= n : m > n;
 }
 
 // The jobs of a mixed call that take the tensor-core sweeps: left-canonical,
 // tall, 64+ columns (their left factor comes from the final columns).
 __host__ __device__ __forceinline__ bool tc_job(int m, int n, int keep_left_canonical) {
-    return !job_tracks_v(m, n, keep_left_canonical) && (m < n ? m : n) >= 64;
+    return keep_left_canonical != 0 && m >= n && n >= 64;
 }
 
 // ... and whose merge runs on the tensor cores as well (theta not given;
@@ -91,6 +106,23 @@ __host__ __device__ __forceinline__ bool tc_job(int m, int n, int keep_left_cano
 __host__ __device__ __forceinline__ bool merge_on_tensor_cores(const mps_2q_job& job, int d) {
     return d <= 4 && tc_job(job.chi_l * d, job.chi_r * d, job.keep_left_canonical) &&
            (job.flags & MPS_JOB_THETA_GIVEN) == 0;
+}
+
+// Column length of a job's slot: the sweep kernels' row steps.
+__host__ __device__ __forceinline__ int slot_rows(int L) {
+    return L <= 64 ? 64 : L <= 128 ? 128 : L <= 256 ? 256 : L <= 512 ? 512 : L <= 576 ? 576
+           : L <= 1024 ? 1024 : L <= 1792 ? 1792 : (L + 31) / 32 * 32;
+}
+
+// The default threshold on a pair's squared cosine for columns of that length.
+// The computed x_p^H x_q carries a rounding error of a few 2^-24
+// sum_r |x_r||q_r|, growing slowly with the length L; tol = 2^-24 max(8,
+// sqrt(L)) stays above that noise (no sweep keeps rotating noise) while the
+// kept subspace -- whose error is about tol s_k / gap at the truncation cut --
+// stays close to what a backward-stable complex64 SVD gives.
+__host__ __device__ __forceinline__ float default_tol2(int rows) {
+    const float tol = 5.9604645e-8f * fmaxf(8.f, sqrtf((float)rows));
+    return tol * tol;
 }
 
 // Singular values at or below this (relative to max(s_0, 1)) are treated as
@@ -104,7 +136,8 @@ int lq_precondition(const mps_2q_job* jobs, int njobs, int max_m, int max_n, con
 
 // One sweep of the SIMT jobs by Gram visits (gramsweep.cu): slots of up to
 // kGramRows rows, blocks of kGramBlock columns; arguments as for jacobi.cu's
-// sweep kernel.
+// sweep kernel, but tol2 = 0 asks for each job's own default (by its own
+// length, so that it does not depend on the jobs it shares the call with).
 constexpr int kGramRows = 1024;
 constexpr int kGramBlock = 8;
 // gram_begin_launch, before each sweep, lists the jobs left in g.gact and clears
