@@ -18,12 +18,11 @@
 //
 // Algorithm: blocked Householder reflectors applied from the right.  For
 // each panel of LQ_B rows k0 .. k0+kb-1:
-//   lq_panel_kernel (one CTA per job): the panel (kb x (C-k0)) in shared
-//     memory; for row i the reflector H_i = I - tau_i v_i v_i^H with
-//     x_i H_i = beta_i e_i (x_i the row, beta_i real; the textbook complex
+//   lq_panel_kernel (one CTA per job), row i's reflector H_i = I - tau_i v_i v_i^H
+//     with x_i H_i = beta_i e_i (x_i the row, beta_i real; the textbook complex
 //     Householder vector of y = x_i^H: beta = -sign(Re y0) |y|,
 //     tau = (beta - y0) / beta, v = (1, y_1.. / (y0 - beta))), applied at once
-//     to the panel rows below; then the compact WY factor
+//     to the panel rows below; and the compact WY factor
 //     H_0 ... H_{kb-1} = I - V T V^H (T upper triangular,
 //     T[0:i, i] = -tau_i T[0:i, 0:i] V[:, 0:i]^H v_i).
 //   lq_trail_kernel (job x 64-row tiles): the rows below the panel,
@@ -33,15 +32,17 @@
 // after the sweeps.
 #include <mutex>
 
+#include "gemm.cuh"
 #include "twoq.cuh"
 
 namespace mps {
 namespace {
 
 constexpr int LQ_B = 32;        // rows per panel
-constexpr int LQ_T = 1024;      // threads of the panel kernel: a warp per panel row
-constexpr int LQ_NW = LQ_T / 32;
+constexpr int LQ_RW = 16;       // warps of the panel kernel, two rows each
+constexpr int LQ_T = LQ_RW * 32;
 constexpr int LQ_TR = 64;       // rows per trailing-update CTA
+constexpr int LQ_TC = 64;       // columns of one step of the trailing update's second product
 constexpr int LQ_MIN_C = 64;    // narrower jobs converge in a few cheap sweeps anyway
 constexpr int LQ_MAX_C = 768;   // the panel (LQ_B x (C+1)) must fit in shared memory
 // V (C x LQ_B) and T (LQ_B x LQ_B, at offset LQ_B * cslot) must fit in the
@@ -57,122 +58,179 @@ __device__ __forceinline__ bool lq_job(const mps_2q_job& job, int d, int& L, int
     return C >= LQ_MIN_C && C <= LQ_MAX_C;
 }
 
-__device__ __forceinline__ cf cinv(cf a) {
-    const float s = 1.f / cabs2(a);
-    return cmake(a.x * s, -a.y * s);
+// Shared memory of the panel kernel for nc columns, in units of cf.
+__host__ __device__ constexpr int panel_stride(int nc) { return nc | 1; }   // odd: no bank conflicts
+__host__ __device__ constexpr size_t panel_elems(int nc, int nt) {
+    return (size_t)LQ_B * panel_stride(nc) + 2 * 32 * nt + LQ_B * LQ_B + LQ_B * (LQ_B + 1) +
+           4 * LQ_B;
 }
 
-__global__ void __launch_bounds__(LQ_T)
+// The four values' sums over the warp, in every lane: halves of the warp take two
+// of them each, then quarters one each (10 shuffles instead of 20).
+__device__ __forceinline__ void warp_sum4(float& v0, float& v1, float& v2, float& v3, int lane) {
+    const bool h = lane & 16, q = lane & 8;
+    const float a = (h ? v2 : v0) + __shfl_xor_sync(0xffffffffu, h ? v0 : v2, 16);
+    const float b = (h ? v3 : v1) + __shfl_xor_sync(0xffffffffu, h ? v1 : v3, 16);
+    float c = (q ? b : a) + __shfl_xor_sync(0xffffffffu, q ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    v0 = __shfl_sync(0xffffffffu, c, 0);
+    v1 = __shfl_sync(0xffffffffu, c, 8);
+    v2 = __shfl_sync(0xffffffffu, c, 16);
+    v3 = __shfl_sync(0xffffffffu, c, 24);
+}
+
+// A panel of at most 32 NT columns.  Its 32 reflectors are a serial chain, so the
+// kernel is bound by a reflector's latency and, beyond ~300 columns, by the FMAs of
+// one SM.  The rows therefore stay in registers (warp w: rows w and w + 16, lane l:
+// columns l, l + 32, ...) and only the pivot row's u_i = v_i (y0 - beta) goes through
+// shared memory, conjugated; one barrier a reflector.  Every row r takes the same
+// product a = x_r u_i: a row below becomes x_r - tau a conj(u_i) / |y0 - beta|^2, and
+// for a row above it is (V^H V)[r][i] up to conj(inv_r) inv_i, which T needs.  The
+// warp of the next pivot row computes its scalars, that of the last one T's column.
+// Mean panel of a 512-column job: 38 us (before, with the rows in shared memory, a
+// warp a row, and T afterwards: 94 us).
+template <int NT>
+__global__ void __launch_bounds__(LQ_T, 1)
 lq_panel_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int k0) {
     extern __shared__ float2 lq_sm[];
     const int j = blockIdx.x;
     int L, C;
     if (!lq_job(jobs[j], g.d, L, C) || k0 >= C) return;
-    const int kb = min(LQ_B, C - k0), nc = C - k0, ps = nc + 1;
+    const int kb = min(LQ_B, C - k0), nc = C - k0, ps = panel_stride(nc);
     cf* P = lq_sm;                              // [kb][ps]: the panel, row-major
-    cf* zz = P + (size_t)LQ_B * ps;             // [LQ_B][LQ_B]: (V^H V)[a][b], a < b
-    cf* Ts = zz + LQ_B * LQ_B;                  // [LQ_B][LQ_B]: T, row-major
-    cf* tau = Ts + LQ_B * LQ_B;                 // [LQ_B]
+    cf* xs = P + (size_t)LQ_B * ps;             // [2][32 NT]: conj(u) of the pivot row
+    cf* zz = xs + 2 * 32 * NT;                  // [LQ_B][LQ_B]: (V^H V)[a][b], a < b (0 else)
+    cf* Ts = zz + LQ_B * LQ_B;                  // [LQ_B][LQ_B + 1]: T, row-major
+    cf* tau = Ts + LQ_B * (LQ_B + 1);           // [LQ_B]
     cf* invs = tau + LQ_B;                      // [LQ_B]: 1 / (y0 - beta)
-    float* betas = reinterpret_cast<float*>(invs + LQ_B);   // [LQ_B]
-    float* tail = betas + LQ_B;                 // [2]: |row i|^2 beyond its diagonal
+    cf* taun = invs + LQ_B;                     // [LQ_B]: tau / |y0 - beta|^2
+    float* betas = reinterpret_cast<float*>(taun + LQ_B);   // [LQ_B]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     cf* X = g.X + (size_t)j * g.lslot * g.cslot;
 
-#pragma unroll 4
-    for (int e = tid; e < kb * nc; e += LQ_T) {
-        const int r = e % kb, c = e / kb;
-        P[r * ps + c] = X[(size_t)(k0 + c) * g.lslot + k0 + r];
-    }
-    __syncthreads();
-    if (warp == 0) {
-        float s = 0.f;
-        for (int c = 1 + lane; c < nc; c += 32) s += cabs2(P[c]);
-        s = warp_sum(s);
-        if (lane == 0) tail[0] = s;
-    }
+    const uint32_t pbase = (uint32_t)__cvta_generic_to_shared(P);
+    for (int c = warp; c < nc; c += LQ_RW)
+        if (lane < kb)
+            copy8_async(pbase + (uint32_t)(lane * ps + c) * 8u,
+                        X + (size_t)(k0 + c) * g.lslot + k0 + lane, 8u);
+    for (int e = tid; e < LQ_B * (2 * LQ_B + 1); e += LQ_T) zz[e] = cmake(0.f, 0.f);   // and T
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 
-    // One barrier per reflector.  Every thread derives H_i from row i's
-    // diagonal entry and tail norm (left by the warp that updated row i in the
-    // step before); the rows below use row i unscaled (v = conj(x) inv), and
-    // row i becomes (beta, v) only after the loop.
-    for (int i = 0; i < kb; ++i) {
-        const cf* x = P + (size_t)i * ps;
-        const cf y0 = cconj(x[i]);
-        const float s = tail[i & 1];
-        cf t = cmake(0.f, 0.f), inv = cmake(0.f, 0.f);
-        float beta = y0.x;
-        if (s > 0.f || y0.y != 0.f) {
-            const float nrm = sqrtf(cabs2(y0) + s);
-            beta = y0.x >= 0.f ? -nrm : nrm;
-            t = cmake((beta - y0.x) / beta, -y0.y / beta);
-            inv = cinv(cmake(y0.x - beta, y0.y));
+    // Row i of this warp's two: its scalars and u.
+    cf z[2][NT];
+    const auto publish = [&](int i) {
+        const int h = i / LQ_RW;
+        float s = 0.f;
+        cf* x = xs + (i & 1) * 32 * NT + lane;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            cf v = h ? z[1][t] : z[0][t];
+            if (t == 0 && lane <= i) v = cmake(0.f, 0.f);
+            s += cabs2(v);
+            x[32 * t] = v;
         }
-        if (tid == 0) {
+        s = warp_sum(s);
+        const cf y = h ? z[1][0] : z[0][0];
+        if (lane == i) {
+            const cf y0 = cconj(y);
+            const float n2 = cabs2(y0) + s;
+            cf t = cmake(0.f, 0.f), inv = cmake(0.f, 0.f), tn = cmake(0.f, 0.f);
+            float beta = y0.x;
+            // (a row whose square is no normal number has no reflector: 1 / |y0 - beta|^2
+            // would overflow)
+            if ((s > 0.f || y0.y != 0.f) && !(n2 < 4.8e-38f)) {
+                const float nrm = sqrtf(n2);
+                beta = y0.x >= 0.f ? -nrm : nrm;
+                const cf u = cmake(y0.x - beta, y0.y);
+                const float rb = 1.f / beta, q = 1.f / cabs2(u);
+                t = cmake(-u.x * rb, -u.y * rb);
+                inv = cmake(u.x * q, -u.y * q);
+                tn = cscale(t, q);
+                *x = cconj(u);
+            }
             tau[i] = t;
             invs[i] = inv;
+            taun[i] = tn;
             betas[i] = beta;
         }
-        // z <- z H_i: d = z v = z[i] + inv sum_c z[c] conj(x[c]);
-        // z[i] -= tau d, z[c] -= tau d conj(inv) x[c]
-        for (int r = i + 1 + warp; r < kb; r += LQ_NW) {
-            cf* z = P + (size_t)r * ps;
-            const cf zi = z[i];
-            cf acc = cmake(0.f, 0.f);
-            for (int c = i + 1 + lane; c < nc; c += 32) cfma_conj(acc, x[c], z[c]);
-            acc.x = warp_sum(acc.x);
-            acc.y = warp_sum(acc.y);
-            const cf td = cmul(t, cadd(zi, cmul(inv, acc)));
-            const cf kx = cmul(td, cconj(inv));
-            if (lane == 0) z[i] = csub(zi, td);
-            float nn = 0.f;
-            for (int c = i + 1 + lane; c < nc; c += 32) {
-                const cf zc = csub(z[c], cmul(kx, x[c]));
-                z[c] = zc;
-                if (c > i + 1) nn += cabs2(zc);
-            }
-            if (r == i + 1) {
-                nn = warp_sum(nn);
-                if (lane == 0) tail[(i + 1) & 1] = nn;
+    };
+    // T[a][b] for all a, from column b of V^H V
+    const auto t_column = [&](int b) {
+        cf s0 = cmake(0.f, 0.f), s1 = cmake(0.f, 0.f);
+        for (int q0 = 0; q0 < b; q0 += 8) {
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) {
+                cfma(s0, Ts[lane * (LQ_B + 1) + q0 + q], zz[(q0 + q) * LQ_B + b]);
+                cfma(s1, Ts[lane * (LQ_B + 1) + q0 + q + 1], zz[(q0 + q + 1) * LQ_B + b]);
             }
         }
-        __syncthreads();
-    }
-    for (int e = tid; e < kb * nc; e += LQ_T) {
-        const int i = e / nc, c = e - (e / nc) * nc;
-        if (c > i) P[(size_t)i * ps + c] = cmul(cconj(P[(size_t)i * ps + c]), invs[i]);
-        else if (c == i) P[(size_t)i * ps + c] = cmake(betas[i], 0.f);
-    }
-    __syncthreads();
+        const cf tb = tau[b], ts = cmul(tb, cadd(s0, s1));
+        __syncwarp();
+        if (lane <= b) Ts[lane * (LQ_B + 1) + b] = lane == b ? tb : cmake(-ts.x, -ts.y);
+        __syncwarp();
+    };
 
-    // (V^H V)[a][b] for a < b, with V[c][a] = 0 (c < a), 1 (c = a), P[a][c] (c > a)
-    for (int pi = warp; pi < kb * kb; pi += LQ_NW) {
-        const int a = pi / kb, b = pi - (pi / kb) * kb;
-        if (a >= b) continue;
-        const cf* va = P + (size_t)a * ps;
-        const cf* vb = P + (size_t)b * ps;
-        cf s = lane == 0 ? cconj(va[b]) : cmake(0.f, 0.f);
-        for (int c = b + 1 + lane; c < nc; c += 32) cfma_conj(s, va[c], vb[c]);
-        s.x = warp_sum(s.x);
-        s.y = warp_sum(s.y);
-        if (lane == 0) zz[a * LQ_B + b] = s;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int r = warp + LQ_RW * h;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const int c = lane + 32 * t;
+            z[h][t] = r < kb && c < nc ? P[r * ps + c] : cmake(0.f, 0.f);
+        }
+    }
+    if (warp == 0) publish(0);
+    for (int i = 0; i < kb; ++i) {
+        __syncthreads();
+        const cf* x = xs + (i & 1) * 32 * NT + lane;
+        cf a0 = cmake(0.f, 0.f), a1 = cmake(0.f, 0.f);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const cf xv = x[32 * t];
+            cfma_conj(a0, xv, z[0][t]);
+            cfma_conj(a1, xv, z[1][t]);
+        }
+        warp_sum4(a0.x, a0.y, a1.x, a1.y, lane);
+        const cf mt = cmake(-taun[i].x, -taun[i].y);
+        const cf w0 = cmul(mt, a0), w1 = cmul(mt, a1);
+        if (warp > i) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const cf xv = x[32 * t];
+                cfma(z[0][t], w0, xv);
+                cfma(z[1][t], w1, xv);
+            }
+        } else if (warp + LQ_RW > i) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t) cfma(z[1][t], w1, x[32 * t]);
+        }
+        if (i + 1 < kb && warp == (i + 1) % LQ_RW) publish(i + 1);
+        if (lane == 0) {
+            const cf inv = invs[i];
+            if (warp < i) zz[warp * LQ_B + i] = cmul(cmul(cconj(invs[warp]), inv), a0);
+            if (warp + LQ_RW < i)
+                zz[(warp + LQ_RW) * LQ_B + i] = cmul(cmul(cconj(invs[warp + LQ_RW]), inv), a1);
+        }
+        if (i > 0 && warp == (i - 1) % LQ_RW) t_column(i - 1);
     }
     __syncthreads();
-    if (warp == 0) {
-        for (int i = 0; i < kb; ++i) {
-            cf val = cmake(0.f, 0.f);
-            if (lane < i) {
-                cf s = cmake(0.f, 0.f);
-                for (int b = lane; b < i; ++b) cfma(s, Ts[lane * LQ_B + b], zz[b * LQ_B + i]);
-                const cf ts = cmul(tau[i], s);
-                val = cmake(-ts.x, -ts.y);
-            } else if (lane == i) {
-                val = tau[i];
-            }
-            __syncwarp();
-            Ts[lane * LQ_B + i] = val;
-            __syncwarp();
+    // the rows to shared memory: L left of the diagonal, beta on it, v right of it
+    if (warp == (kb - 1) % LQ_RW) t_column(kb - 1);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int r = warp + LQ_RW * h;
+        if (r >= kb) continue;
+        const cf inv = invs[r];
+        const float beta = betas[r];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const int c = lane + 32 * t;
+            cf v = z[h][t];
+            if (t > 0 || lane > r) v = cmul(cconj(v), inv);
+            else if (lane == r) v = cmake(beta, 0.f);
+            if (c < nc) P[r * ps + c] = v;
         }
     }
     __syncthreads();
@@ -183,142 +241,133 @@ lq_panel_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int k0) {
     for (int e = tid; e < nc * LQ_B; e += LQ_T) {
         const int c = e / LQ_B, b = e % LQ_B;
         cf v = cmake(0.f, 0.f);
-        if (b < kb) v = c < b ? cmake(0.f, 0.f) : (c == b ? cmake(1.f, 0.f) : P[(size_t)b * ps + c]);
+        if (b < kb) v = c < b ? cmake(0.f, 0.f) : (c == b ? cmake(1.f, 0.f) : P[b * ps + c]);
         Vg[e] = v;
     }
     for (int e = tid; e < LQ_B * LQ_B; e += LQ_T) {
         const int a = e / LQ_B, b = e % LQ_B;
-        Tg[e] = (a < kb && b < kb && b >= a) ? Ts[e] : cmake(0.f, 0.f);
+        Tg[e] = a < kb && b < kb && b >= a ? Ts[a * (LQ_B + 1) + b] : cmake(0.f, 0.f);
     }
-    // the panel's rows of L: left of the diagonal as transformed, beta on it,
-    // zero right of it
-    for (int e = tid; e < kb * nc; e += LQ_T) {
-        const int r = e % kb, c = e / kb;
-        const cf v = c <= r ? P[r * ps + c] : cmake(0.f, 0.f);
-        X[(size_t)(k0 + c) * g.lslot + k0 + r] = v;
-    }
+    // the panel's rows of L: zero right of the diagonal
+    for (int c = warp; c < nc; c += LQ_RW)
+        if (lane < kb)
+            X[(size_t)(k0 + c) * g.lslot + k0 + lane] =
+                c <= lane ? P[lane * ps + c] : cmake(0.f, 0.f);
 }
 
-// Rows k0+kb .. L-1 of the job: R <- R - ((R V) T) V^H, 64 rows per CTA,
-// in 32-column chunks; each chunk's global loads are issued while the
-// previous chunk is being multiplied.
-__global__ void __launch_bounds__(256)
+// Rows k0+kb .. L-1 of the job, 64 per CTA: W = R V by the shared GEMM tile, W T
+// in shared memory, then R - (W T) V^H in steps of 64 columns with V's rows and R's
+// entries fetched a step ahead.  Both products read shared memory in 8 wavefronts
+// for 64 FMAs a thread, so the FP32 pipes bound it: mean launch of 63 jobs of 512
+// columns 47 us (73 us before, when the second product read 3 wavefronts for
+// every 4 FMAs).
+struct TrailSmem {
+    using Tile = GemmTile<LQ_TR, LQ_B, 2>;
+    static constexpr int VST = LQ_TC + 1;
+    union {
+        cf ab[Tile::ST * Tile::BUF];            // the first product's chunks
+        cf vt[2][LQ_B][VST];                    // a step's 64 rows of V, transposed
+    };
+    cf w[LQ_B][LQ_TR + 1];                      // W, then W T
+    cf t[LQ_B][LQ_B];
+};
+
+__global__ void __launch_bounds__(256, 2)
 lq_trail_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int k0) {
-    // phase 1: Xs [32][LQ_TR] and Bs [32][LQ_B] (a V chunk, then T);
-    // phase 2: Vt [LQ_B][33] (a conjugated V chunk, transposed) over Xs
-    __shared__ cf sm[32 * LQ_TR + 32 * LQ_B + LQ_B * LQ_TR];
-    cf (*Xs)[LQ_TR] = reinterpret_cast<cf (*)[LQ_TR]>(sm);
-    cf (*Vt)[33] = reinterpret_cast<cf (*)[33]>(sm);
-    cf (*Bs)[LQ_B] = reinterpret_cast<cf (*)[LQ_B]>(sm + 32 * LQ_TR);
-    cf (*Ws)[LQ_TR] = reinterpret_cast<cf (*)[LQ_TR]>(sm + 32 * LQ_TR + 32 * LQ_B);
+    extern __shared__ float2 lq_sm[];
+    TrailSmem& sm = *reinterpret_cast<TrailSmem*>(lq_sm);
     const int j = blockIdx.y;
     int L, C;
     if (!lq_job(jobs[j], g.d, L, C) || k0 >= C) return;
     const int kb = min(LQ_B, C - k0), nc = C - k0;
     const int row0 = k0 + kb + blockIdx.x * LQ_TR;
     if (row0 >= L) return;
-    const int tid = threadIdx.x, rr = tid & (LQ_TR - 1), q = tid / LQ_TR;   // q: 0..3
-    const int r = row0 + rr;
-    const bool live = r < L;
-    cf* X = g.X + (size_t)j * g.lslot * g.cslot;
+    const int tid = threadIdx.x, rows = L - row0;
+    cf* R = g.X + (size_t)j * g.lslot * g.cslot + (size_t)k0 * g.lslot + row0;
     const cf* Vg = g.V + (size_t)j * g.cslot * g.cslot;
     const cf* Tg = Vg + (size_t)LQ_B * g.cslot;
-    const cf zero = cmake(0.f, 0.f);
 
-    // W[r][b] = sum_c X[r][k0 + c] V[c][b]; this thread: b = q*8 .. q*8+7.
-    // Staging: element q2*256 + tid of a chunk is X column q2*4 + q, row rr,
-    // and V row (q2*256+tid)/32, column tid % 32.
-    cf xr[8], vr[4];
-    auto fetch1 = [&](int c0) {
+    for (int e = tid; e < LQ_B * LQ_B; e += 256) (&sm.t[0][0])[e] = Tg[e];
+    const GemmArgs a{min(rows, LQ_TR), LQ_B, nc, R, 1, g.lslot, 0, Vg, LQ_B, 1, 0, nullptr, 0, 0};
+    for (int e = tid; e < LQ_B * (LQ_TR + 1); e += 256) (&sm.w[0][0])[e] = cmake(0.f, 0.f);
+    __syncthreads();
+    TrailSmem::Tile::run<false, false>(a, 0, 0, nullptr, sm.ab,
+                                       [&](int r, int b, cf v) { sm.w[b][r] = v; });
+    __syncthreads();
+    const uint32_t vbase = (uint32_t)__cvta_generic_to_shared(&sm.vt[0][0][0]);
+    const auto fetch_v = [&](int c0) {
+        const uint32_t off = vbase + (uint32_t)((c0 / LQ_TC) & 1) * (LQ_B * TrailSmem::VST * 8);
 #pragma unroll
-        for (int q2 = 0; q2 < 8; ++q2) {
-            const int c = c0 + q2 * 4 + q;
-            xr[q2] = (c < nc && live) ? X[(size_t)(k0 + c) * g.lslot + r] : zero;
+        for (int q = 0; q < LQ_TC * LQ_B / 256; ++q) {
+            const int e = tid + 256 * q, c = e / LQ_B, b = e % LQ_B;
+            const bool in = c0 + c < nc;
+            copy8_async(off + (uint32_t)(b * TrailSmem::VST + c) * 8u,
+                        in ? Vg + (size_t)(c0 + c) * LQ_B + b : Vg, in ? 8u : 0u);
         }
-#pragma unroll
-        for (int q2 = 0; q2 < 4; ++q2) {
-            const int e = q2 * 256 + tid, c = c0 + e / LQ_B;
-            vr[q2] = c < nc ? Vg[(size_t)c * LQ_B + (e % LQ_B)] : zero;
-        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    cf acc[8];
+    fetch_v(0);
+    // W <- W T (T upper triangular): row r, columns q, q + 4, ...
+    {
+        const int r = tid & (LQ_TR - 1), q = tid / LQ_TR;
+        cf w[LQ_B / 4];
 #pragma unroll
-    for (int b = 0; b < 8; ++b) acc[b] = zero;
-    fetch1(0);
-    for (int c0 = 0; c0 < nc; c0 += 32) {
-#pragma unroll
-        for (int q2 = 0; q2 < 8; ++q2) Xs[q2 * 4 + q][rr] = xr[q2];
-#pragma unroll
-        for (int q2 = 0; q2 < 4; ++q2) {
-            const int e = q2 * 256 + tid;
-            Bs[e / LQ_B][e % LQ_B] = vr[q2];
-        }
-        __syncthreads();
-        if (c0 + 32 < nc) fetch1(c0 + 32);
+        for (int e = 0; e < LQ_B / 4; ++e) w[e] = cmake(0.f, 0.f);
 #pragma unroll 4
-        for (int cc = 0; cc < 32; ++cc) {
-            const cf x = Xs[cc][rr];
+        for (int i = 0; i < LQ_B; ++i) {
+            const cf x = sm.w[i][r];
 #pragma unroll
-            for (int b = 0; b < 8; ++b) cfma(acc[b], x, Bs[cc][q * 8 + b]);
+            for (int e = 0; e < LQ_B / 4; ++e) cfma(w[e], x, sm.t[i][q + 4 * e]);
         }
         __syncthreads();
+#pragma unroll
+        for (int e = 0; e < LQ_B / 4; ++e) sm.w[q + 4 * e][r] = cmake(-w[e].x, -w[e].y);
     }
-    // W <- W T (T upper triangular)
+    // this thread: rows tx + 16 i, columns ty + 16 j of a step
+    const int tx = tid & 15, ty = tid >> 4;
+    cf zr[4][4];
+    const auto fetch_r = [&](int c0) {
 #pragma unroll
-    for (int b = 0; b < 8; ++b) Ws[q * 8 + b][rr] = acc[b];
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int q2 = 0; q2 < 4; ++q2) {
-        const int e = q2 * 256 + tid;
-        Bs[e / LQ_B][e % LQ_B] = Tg[e];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        const int bb = q * 8 + b;
-        cf w = zero;
-        for (int a = 0; a <= bb; ++a) cfma(w, Ws[a][rr], Bs[a][bb]);
-        acc[b] = w;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < 8; ++b) Ws[q * 8 + b][rr] = acc[b];
-
-    // X[r][k0 + c] -= sum_b W[r][b] conj(V[c][b]); this thread: columns
-    // q*8 .. q*8+7 of each chunk (its row's entries fetched a chunk ahead)
-    cf zr[8];
-    auto fetch2 = [&](int c0) {
-#pragma unroll
-        for (int q2 = 0; q2 < 4; ++q2) {
-            const int e = q2 * 256 + tid, c = c0 + e / LQ_B;
-            vr[q2] = c < nc ? Vg[(size_t)c * LQ_B + (e % LQ_B)] : zero;
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int c = c0 + q * 8 + k;
-            zr[k] = (live && c < nc) ? X[(size_t)(k0 + c) * g.lslot + r] : zero;
-        }
+            for (int q = 0; q < 4; ++q) {
+                const int r = tx + 16 * i, c = c0 + ty + 16 * q;
+                zr[i][q] = r < rows && c < nc ? R[(size_t)c * g.lslot + r] : cmake(0.f, 0.f);
+            }
     };
-    fetch2(0);
-    for (int c0 = 0; c0 < nc; c0 += 32) {
+    fetch_r(0);
+    for (int c0 = 0; c0 < nc; c0 += LQ_TC) {
+        cf acc[4][4];
 #pragma unroll
-        for (int q2 = 0; q2 < 4; ++q2) {
-            const int e = q2 * 256 + tid;
-            Vt[e % LQ_B][e / LQ_B] = cconj(vr[q2]);
-        }
-        cf z[8];
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) z[k] = zr[k];
+            for (int q = 0; q < 4; ++q) acc[i][q] = zr[i][q];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (c0 + 32 < nc) fetch2(c0 + 32);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int cc = q * 8 + k, c = c0 + cc;
-            cf s = cmake(0.f, 0.f);
+        if (c0 + LQ_TC < nc) {
+            fetch_v(c0 + LQ_TC);
+            fetch_r(c0 + LQ_TC);
+        }
+        const cf (*vt)[TrailSmem::VST] = sm.vt[(c0 / LQ_TC) & 1];
 #pragma unroll 8
-            for (int b = 0; b < LQ_B; ++b) cfma(s, Ws[b][rr], Vt[b][cc]);
-            if (live && c < nc) X[(size_t)(k0 + c) * g.lslot + r] = csub(z[k], s);
+        for (int b = 0; b < LQ_B; ++b) {
+            cf wv[4], vv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) wv[i] = sm.w[b][tx + 16 * i];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) vv[q] = vt[b][ty + 16 * q];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) cfma_conj(acc[i][q], vv[q], wv[i]);
         }
-        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = tx + 16 * i, c = c0 + ty + 16 * q;
+                if (r < rows && c < nc) R[(size_t)c * g.lslot + r] = acc[i][q];
+            }
     }
 }
 
@@ -347,22 +396,34 @@ int lq_precondition(const mps_2q_job* jobs, int njobs, int max_m, int max_n, con
     // the shared-memory opt-in is per device: set it once on every device used
     static std::once_flag once[kMaxDevices];
     static cudaError_t attr[kMaxDevices];
-    const size_t smem_max = ((size_t)LQ_B * (LQ_MAX_C + 1) + 2 * LQ_B * LQ_B + 3 * LQ_B) * sizeof(cf);
+    // kernels for panels of up to 64, 128, 256, 384, ... columns
+    static constexpr int kNt[] = {2, 4, 8, 12, 16, 20, 24};
+    static void (*const kPanel[])(const mps_2q_job*, TwoQGeom, int) = {
+        lq_panel_kernel<2>,  lq_panel_kernel<4>,  lq_panel_kernel<8>, lq_panel_kernel<12>,
+        lq_panel_kernel<16>, lq_panel_kernel<20>, lq_panel_kernel<24>};
     int dev = 0;
     MPS_CUDA_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kMaxDevices) return fail(MPS_ERR_ARG, "lq_precondition: device index beyond 63");
     std::call_once(once[dev], [&] {
-        attr[dev] = cudaFuncSetAttribute(lq_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_max);
+        attr[dev] = cudaSuccess;
+        for (int q = 0; q < 7 && attr[dev] == cudaSuccess; ++q)
+            attr[dev] = cudaFuncSetAttribute(kPanel[q], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(panel_elems(32 * kNt[q], kNt[q]) * sizeof(cf)));
+        if (attr[dev] == cudaSuccess)
+            attr[dev] = cudaFuncSetAttribute(lq_trail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(TrailSmem));
     });
     if (attr[dev] != cudaSuccess) return cuda_fail(attr[dev], "cudaFuncSetAttribute(lq_panel_kernel)");
-    const size_t smem = ((size_t)LQ_B * (cmax + 1) + 2 * LQ_B * LQ_B + 3 * LQ_B) * sizeof(cf);
     for (int k0 = 0; k0 < cmax; k0 += LQ_B) {
-        lq_panel_kernel<<<njobs, LQ_T, smem, s>>>(jobs, g, k0);
+        int q = 0;
+        while (32 * kNt[q] < cmax - k0) ++q;
+        const size_t smem = panel_elems(cmax - k0, kNt[q]) * sizeof(cf);
+        kPanel[q]<<<njobs, LQ_T, smem, s>>>(jobs, g, k0);
         MPS_LAUNCH_CHECK("lq_panel_kernel");
         const int rows = max(max_m, max_n) - k0;   // covers every job's rows below its panel
         if (rows > 0) {
-            lq_trail_kernel<<<dim3((rows + LQ_TR - 1) / LQ_TR, njobs), 256, 0, s>>>(jobs, g, k0);
+            lq_trail_kernel<<<dim3((rows + LQ_TR - 1) / LQ_TR, njobs), 256, sizeof(TrailSmem), s>>>(
+                jobs, g, k0);
             MPS_LAUNCH_CHECK("lq_trail_kernel");
         }
     }
