@@ -39,11 +39,16 @@
 // once: one CTA per SM whose warps are specialised -- a loader (claims items,
 // waits for their blocks, brings the columns in by bulk copies), Gram warps, one
 // solver warp per visit slot, and apply warps -- and pass S visit slots round in
-// order through mbarriers.
+// order through mbarriers.  The columns themselves lie in B <= S buffers of their
+// own: once the apply warps hold a visit's rows in registers its buffer takes the
+// next visit's columns, while the rotations and the write-back go on.
 //
 // Measured (GB300): 32 theta of 512 x 512, mean sweep 1.21 ms against 1.76 of the
-// column-by-column kernel, an SM 10.8K cycles a visit (FMA work 3.2K; three slots
-// of 66 KB fill shared memory, so a visit's latency, ~30K cycles, bounds it); 24
+// column-by-column kernel (57% of the issue slots busy at four warps a scheduler;
+// L2 26%).  Buffers apart from the slots, against a slot that kept its columns to
+// the end: layers of 40 sites chi=420 (one buffer of 1024 rows) 58.3 -> 51.7 ms, of
+// 32 qutrits chi=192 14.75 -> 14.3, of 64 sites chi=256 19.8 -> 19.4; slots of up to
+// 256 rows have a buffer each (sharing them measured 1-3% slower).  24
 // of 256 x 256, 0.26 against 0.29 ms; wide or right-canonical jobs of 200
 // columns (V rows included), 0.24 against 0.35 ms.  Variants measured on the
 // same case (512 x 512): 16-column blocks with four solver warps, 1.9 ms; three
@@ -65,7 +70,8 @@ constexpr int GS_GST = GS_W + 1;             // row stride of G in shared memory
 constexpr int GS_FULL = GS_W - 1;            // steps of a full visit
 constexpr int GS_NP = GS_BC * GS_BC;         // products of two blocks
 constexpr int GS_NBLK = GS_BC * (GS_BC - 1) / 2;   // 2 x 2 blocks off the diagonal
-constexpr int GS_LEAD = 1;                   // steps the solver is ahead when a warp starts
+constexpr int GS_LEAD = 3;                   // step the solver has taken when a warp starts
+                                             // (1 where each slot has its own buffer)
 constexpr int GS_TRIES = 1 << 20;            // suspended tries of a slot wait
 constexpr unsigned GS_SUSPEND_NS = 1000;
 constexpr float kInnerTol2 = 0.25f;
@@ -90,6 +96,7 @@ struct Slot {
     float scale[GS_W];                       // the columns' scales at the end, less 1
     alignas(8) unsigned mask[GS_W];          // pairs that rotate in a step
     int col[GS_W];                           // physical columns
+    int buf;                                 // the column buffer
     int job, I, J, full, L, vrows;
     float tol2;        // the visit (job < 0: no more)
     int time, changedI, changedJ;            // its time, when its blocks last changed
@@ -101,9 +108,9 @@ struct Slot {
     uint64_t b_ring[GS_BC], b_circle[GS_FULL];
 };
 
-template <int LW, int S, int NG>
+template <int LW, int B, int S, int NG>
 constexpr size_t gs_smem() {
-    return S * ((size_t)GS_W * (LW + 2) * sizeof(cf) + sizeof(Slot<NG>));
+    return B * ((size_t)GS_W * (LW + 2) * sizeof(cf) + sizeof(uint64_t) * 2) + S * sizeof(Slot<NG>);
 }
 
 // Column blocks of a job of C columns: an even number, two at least.
@@ -194,13 +201,12 @@ template <int XST, int NG>
 __device__ __forceinline__ void gram_partial(const cf* Xs, int a0, int b0, int L, cf* part,
                                              float* pn, int warp, int lane) {
     const int grp = lane >> 2, ti = (lane >> 1) & 1, tj = lane & 1;
-    const float4* xa[4];
-    const float4* xb[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        xa[c] = reinterpret_cast<const float4*>(Xs + (size_t)(a0 + 4 * ti + ((c + 2 * tj) & 3)) * XST);
-        xb[c] = reinterpret_cast<const float4*>(Xs + (size_t)(b0 + 4 * tj + ((c + 2 * ti) & 3)) * XST);
-    }
+    constexpr int CST = XST / 2;              // a column in row pairs
+    const float4* x4 = reinterpret_cast<const float4*>(Xs);
+    const float4* xa0 = x4 + (a0 + 4 * ti + 2 * tj) * CST;
+    const float4* xa2 = x4 + (a0 + 4 * ti + 2 - 2 * tj) * CST;
+    const float4* xb0 = x4 + (b0 + 4 * tj + 2 * ti) * CST;
+    const float4* xb2 = x4 + (b0 + 4 * tj + 2 - 2 * ti) * CST;
     f2 s1[16], s2[16], na[2], nb[2];
 #pragma unroll
     for (int e = 0; e < 16; ++e) s1[e] = s2[e] = 0ull;
@@ -210,7 +216,7 @@ __device__ __forceinline__ void gram_partial(const cf* Xs, int a0, int b0, int L
     for (int rp = 8 * warp + grp; rp < nrp; rp += 8 * NG) {
         float4 y[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) y[c] = xb[c][rp];
+        for (int c = 0; c < 4; ++c) y[c] = (c < 2 ? xb0 + c * CST : xb2 + (c - 2) * CST)[rp];
         f2 ya[4], yb[4], yas[4], ybs[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -221,7 +227,8 @@ __device__ __forceinline__ void gram_partial(const cf* Xs, int a0, int b0, int L
         }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(xa[c] + rp);
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(
+                (c < 2 ? xa0 + c * CST : xa2 + (c - 2) * CST) + rp);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 s1[4 * c + e] = fma2(x.x, ya[e], s1[4 * c + e]);
@@ -544,9 +551,9 @@ struct Turn {
 // of this is a round trip to L2 (the visit slots leave L1 next to nothing), so
 // the next item is claimed and its job looked up while the present one is on
 // its way.
-template <int LW, int S, int NG>
+template <int LW, int B, int S, int NG>
 __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const SweepSync& sync,
-                                       int tbase, cf* Xs,
+                                       int tbase, cf* Xs, uint64_t* b_read,
                                        Slot<NG>* slots, int lane) {
     constexpr int XST = LW + 2;
     const int4 head = __ldcg(g.gact);         // jobs left, their rounds and pairs
@@ -554,6 +561,7 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
     const int total = rounds * per_round;
     volatile int* err = sync.error;
     Turn<S> t;
+    Turn<B> tb;
     bool expired = false;
     int left = S;                             // end markers to post
     const auto claim = [&]() {                // lane 0: the next item, lane 1: the stop flag
@@ -657,10 +665,12 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
                 mbar_arrive(&sl.b_full);
             }
         } else {
+            if (B < S && tb.use > 0) slot_wait(b_read + tb.slot, tb.parity() ^ 1u, expired);
             const uint32_t bytes = (uint32_t)((L + 63) >> 6) * 64u * (uint32_t)sizeof(cf);
             if (lane < GS_W) sl.col[lane] = col;
             if (lane == 0) {
                 sl.job = j;
+                sl.buf = B < S ? tb.slot : t.slot;
                 sl.I = I;
                 sl.J = J;
                 sl.full = r == 0 ? 1 : 0;
@@ -682,9 +692,10 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
             // the bulk copies' (async) reads
             asm volatile("fence.proxy.async;" ::: "memory");
             if (lane < GS_W)
-                tc::bulk_g2s(Xs + ((size_t)t.slot * GS_W + lane) * XST,
+                tc::bulk_g2s(Xs + ((size_t)(B < S ? tb.slot : t.slot) * GS_W + lane) * XST,
                              g.X + (size_t)j * g.lslot * g.cslot + (size_t)col * g.lslot, bytes,
                              &sl.b_full);
+            tb.next();
         }
         t.next();
     }
@@ -702,7 +713,7 @@ __device__ __forceinline__ void gram_role(const SweepSync& sync, const cf* Xs, S
         slot_wait(&sl.b_full, t.parity(), expired);
         if (sl.job < 0 || expired) break;
         const int L = sl.L, np = sl.full ? 3 : 1;
-        const cf* X = Xs + (size_t)t.slot * GS_W * XST;
+        const cf* X = Xs + (size_t)sl.buf * GS_W * XST;
         // inter-block, then (full visits) the two blocks' own
 #pragma unroll 1
         for (int ps = 0; ps < np; ++ps)
@@ -814,9 +825,9 @@ __device__ __forceinline__ void solver_role(const TwoQGeom& g, const SweepSync& 
     if (expired && lane == 0) atomicExch(sync.error, 1);
 }
 
-template <int LW, int S, int NG, int NA>
+template <int LW, int B, int S, int NG, int NA>
 __device__ __forceinline__ void apply_role(const TwoQGeom& g, const SweepSync& sync, const cf* Xs,
-                                           Slot<NG>* slots, int aw, int lane) {
+                                           uint64_t* b_read, Slot<NG>* slots, int aw, int lane) {
     constexpr int XST = LW + 2;
     Turn<S> t;
     bool expired = false;
@@ -827,6 +838,7 @@ __device__ __forceinline__ void apply_role(const TwoQGeom& g, const SweepSync& s
         slot_wait(&sl.b_work, t.parity(), expired);
         const int j = sl.job;
         if (j < 0 || expired) break;
+        bool reading = B < S;                 // the visit's column buffer
         if (sl.work) {
             // tasks of 64 rows, dealt to the warps in turn across visits: the
             // rows of X, then (where the job accumulates it) those of V
@@ -835,12 +847,14 @@ __device__ __forceinline__ void apply_role(const TwoQGeom& g, const SweepSync& s
             const int xp = (sl.L + 63) >> 6, np = xp + ((sl.vrows + 63) >> 6);
             cf* X = g.X + (size_t)j * g.lslot * g.cslot;
             cf* V = g.V + (size_t)j * g.cslot * g.cslot;
-            const cf* Y = Xs + (size_t)t.slot * GS_W * XST;
+            const cf* Y = Xs + (size_t)sl.buf * GS_W * XST;
             int q = first;
             // A warp that followed the solver from its first step would spend
             // the whole solve on one visit; from here on it keeps up with the
-            // steps as they come.
-            if (q < np) slot_wait(full ? sl.b_circle + GS_FULL / 2 : sl.b_ring + GS_LEAD, par, expired);
+            // steps as they come.  (Where a buffer waits for it, the warp takes
+            // the columns first.)
+            uint64_t* start = full ? sl.b_circle + GS_FULL / 2 : sl.b_ring + (B < S ? GS_LEAD : 1);
+            if (B == S && q < np) slot_wait(start, par, expired);
 #pragma unroll 1
             for (; q < np; q += NA) {
                 const bool in_x = q < xp;
@@ -859,6 +873,14 @@ __device__ __forceinline__ void apply_role(const TwoQGeom& g, const SweepSync& s
                         y[c] = make_row2(__ldcg(reinterpret_cast<const float4*>(
                             base + (size_t)sl.col[c] * ld - (live ? 0 : r))));
                 }
+                // this warp's last rows of X are in registers: the buffer's next
+                // columns may come
+                if (reading && q + NA >= xp) {
+                    __syncwarp();
+                    lane0_arrive(b_read + sl.buf, lane);
+                    reading = false;
+                }
+                if (B < S && q == first) slot_wait(start, par, expired);
                 if (full) apply_full(y, sl, par, expired);
                 else apply_ring(y, sl, par, expired);
 #pragma unroll
@@ -874,18 +896,22 @@ __device__ __forceinline__ void apply_role(const TwoQGeom& g, const SweepSync& s
             else par_ring ^= 1u << t.slot;
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sl.b_done);
+        if (lane == 0) {
+            if (reading) mbar_arrive(b_read + sl.buf);
+            mbar_arrive(&sl.b_done);
+        }
     }
     if (expired && lane == 0) atomicExch(sync.error, 1);
 }
 
-template <int LW, int S, int NG, int NA>
+template <int LW, int B, int S, int NG, int NA>
 __global__ void __launch_bounds__((NA + NG + S + 1) * 32, 1)
 gram_sweep_kernel(TwoQGeom g, float tol2, SweepSync sync, int tbase) {
     extern __shared__ __align__(16) float2 gs_sm[];
     if (__ldcg(&g.gact[0].x) == 0) return;    // no job left to sweep here
     cf* Xs = gs_sm;
-    Slot<NG>* slots = reinterpret_cast<Slot<NG>*>(Xs + (size_t)S * GS_W * (LW + 2));
+    Slot<NG>* slots = reinterpret_cast<Slot<NG>*>(Xs + (size_t)B * GS_W * (LW + 2));
+    uint64_t* b_read = reinterpret_cast<uint64_t*>(slots + S);       // buffers read out
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < S) {
         Slot<NG>& sl = slots[warp];
@@ -901,12 +927,16 @@ gram_sweep_kernel(TwoQGeom g, float tol2, SweepSync sync, int tbase) {
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
+    if (B < S && warp == S && lane < B) {
+        mbar_init(b_read + lane, NA);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     __syncthreads();
     const int role = (int)(blockDim.x >> 5) - 1 - warp;          // apply warps first
-    if (role == 0) loader<LW, S, NG>(g, tol2, sync, tbase, Xs, slots, lane);
+    if (role == 0) loader<LW, B, S, NG>(g, tol2, sync, tbase, Xs, b_read, slots, lane);
     else if (role <= S) solver_role<LW, S, NG>(g, sync, slots[role - 1], lane);
     else if (role <= S + NG) gram_role<LW, S, NG>(sync, Xs, slots, role - 1 - S, lane);
-    else apply_role<LW, S, NG, NA>(g, sync, Xs, slots, role - 1 - S - NG, lane);
+    else apply_role<LW, B, S, NG, NA>(g, sync, Xs, b_read, slots, role - 1 - S - NG, lane);
 }
 
 // The jobs left (not done, and not the tensor-core sweeps' in a mixed call), in
@@ -978,11 +1008,11 @@ gram_begin_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs, Sw
     }
 }
 
-template <int LW, int S, int NG, int NA>
+template <int LW, int B, int S, int NG, int NA>
 int launch(int njobs, int rounds, int pairs, const TwoQGeom& g, float tol2, const SweepSync& sync,
            int tbase, cudaStream_t s) {
     static KernelSetup ks;
-    constexpr size_t smem = gs_smem<LW, S, NG>();
+    constexpr size_t smem = gs_smem<LW, B, S, NG>();
     constexpr int threads = (NA + NG + S + 1) * 32;
     static_assert(smem <= 227 * 1024, "visit slots exceed shared memory");
     int dev = 0;
@@ -990,7 +1020,7 @@ int launch(int njobs, int rounds, int pairs, const TwoQGeom& g, float tol2, cons
     if (dev < 0 || dev >= kMaxDevices) return fail(MPS_ERR_ARG, "device index beyond 63");
     std::call_once(ks.once[dev], [&] {
         int rc = MPS_OK, sms = 0;
-        auto kernel = gram_sweep_kernel<LW, S, NG, NA>;
+        auto kernel = gram_sweep_kernel<LW, B, S, NG, NA>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1002,7 +1032,7 @@ int launch(int njobs, int rounds, int pairs, const TwoQGeom& g, float tol2, cons
     const int items = njobs * pairs;          // a round's visits
     const int grid = items < ks.ctas[dev] ? items : ks.ctas[dev];
     if (grid <= 0 || rounds <= 0) return MPS_OK;
-    gram_sweep_kernel<LW, S, NG, NA><<<grid, threads, smem, s>>>(g, tol2, sync, tbase);
+    gram_sweep_kernel<LW, B, S, NG, NA><<<grid, threads, smem, s>>>(g, tol2, sync, tbase);
     MPS_LAUNCH_CHECK("gram_sweep_kernel");
     return MPS_OK;
 }
@@ -1022,12 +1052,12 @@ int gram_sweep_launch(int njobs, int rounds, int pairs, const TwoQGeom& g,
     // (three Gram warps everywhere: a product's partial sums, and so its rounding,
     // do not depend on the slot a job happens to share with others)
     switch (g.lslot) {
-        case 64: return launch<64, 4, 3, 4>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
-        case 128: return launch<128, 4, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
-        case 256: return launch<256, 4, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
-        case 512: return launch<512, 3, 3, 9>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
-        case 576: return launch<576, 2, 3, 10>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
-        case 1024: return launch<1024, 1, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 64: return launch<64, 4, 4, 3, 4>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 128: return launch<128, 4, 4, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 256: return launch<256, 4, 4, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 512: return launch<512, 3, 4, 3, 8>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 576: return launch<576, 2, 3, 3, 9>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
+        case 1024: return launch<1024, 1, 2, 3, 10>(njobs, rounds, pairs, g, tol2, sync, tbase, s);
         default: return fail(MPS_ERR_ARG, "gram sweeps: unsupported slot size");
     }
 }

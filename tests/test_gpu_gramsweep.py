@@ -40,3 +40,19 @@ def test_mixed_shapes_in_one_call(built_lib, cuda):
     assert rc == 0, _native.last_error()
     for spec, out in zip(specs, res):
         check_job(spec, out, 2)
+
+
+@pytest.mark.parametrize("chil,chir", [(255, 256), (288, 280), (289, 150), (512, 200)])
+@pytest.mark.parametrize("lc", [True, False])
+def test_buffers_fewer_than_slots(built_lib, cuda, chil, chir, lc):
+    """The longest slots (512, 576 and 1024 rows), where several visits pass through
+    one column buffer; right-canonical: V rows beside it."""
+    rng = np.random.default_rng(7000 * chil + chir)
+    specs = []
+    for _ in range(3):
+        a, b, g = make_job_inputs(rng, chil, chir, chir, 2, scale=1.0 / chir)
+        specs.append((a, b, g, chir, lc))
+    rc, res, _ = run_batch(built_lib, cuda, specs)
+    assert rc == 0, _native.last_error()
+    for spec, out in zip(specs, res):
+        check_job(spec, out, 2)
