@@ -72,6 +72,7 @@ constexpr int GS_NP = GS_BC * GS_BC;         // products of two blocks
 constexpr int GS_NBLK = GS_BC * (GS_BC - 1) / 2;   // 2 x 2 blocks off the diagonal
 constexpr int GS_LEAD = 3;                   // step the solver has taken when a warp starts
                                              // (1 where each slot has its own buffer)
+constexpr int GS_ACT = 256;                  // jobs left that a CTA keeps in shared memory
 constexpr int GS_TRIES = 1 << 20;            // suspended tries of a slot wait
 constexpr unsigned GS_SUSPEND_NS = 1000;
 constexpr float kInnerTol2 = 0.25f;
@@ -110,7 +111,8 @@ struct Slot {
 
 template <int LW, int B, int S, int NG>
 constexpr size_t gs_smem() {
-    return B * ((size_t)GS_W * (LW + 2) * sizeof(cf) + sizeof(uint64_t) * 2) + S * sizeof(Slot<NG>);
+    return B * ((size_t)GS_W * (LW + 2) * sizeof(cf) + sizeof(uint64_t) * 2) + S * sizeof(Slot<NG>) +
+           GS_ACT * sizeof(int4);
 }
 
 // Column blocks of a job of C columns: an even number, two at least.
@@ -462,10 +464,15 @@ __device__ __forceinline__ int2 ld_state(const int2* p) {
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return make_int2((int)(unsigned)v, (int)(unsigned)(v >> 32));
 }
-__device__ __forceinline__ void st_state(int2* p, int t, int changed) {
-    const unsigned long long v = (unsigned long long)(unsigned)t |
-                                 ((unsigned long long)(unsigned)changed << 32);
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+// (lane 0 writes block I's word, lane 1 block J's, behind one fence)
+__device__ __forceinline__ void st_states(int2* bst, int I, int J, int t, int cI, int cJ, int lane) {
+    if (lane < 2) {
+        const unsigned long long v = (unsigned long long)(unsigned)t |
+                                     ((unsigned long long)(unsigned)(lane ? cJ : cI) << 32);
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(bst + (lane ? J : I)), "l"(v)
+                     : "memory");
+    }
 }
 
 // Waits for a barrier's phase; gives up for good after GS_TRIES suspended tries
@@ -553,7 +560,7 @@ struct Turn {
 // its way.
 template <int LW, int B, int S, int NG>
 __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const SweepSync& sync,
-                                       int tbase, cf* Xs, uint64_t* b_read,
+                                       int tbase, cf* Xs, uint64_t* b_read, const int4* act,
                                        Slot<NG>* slots, int lane) {
     constexpr int XST = LW + 2;
     const int4 head = __ldcg(g.gact);         // jobs left, their rounds and pairs
@@ -576,13 +583,32 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
     // 15.7 against 15.3).
     const bool ahead = per_round > 6 * (int)gridDim.x;
     int claimed = 0, item = 0;
+    int round = 0, round_at = 0, pair = 0;    // the item's round, that round's first item, its pair
+    const float per_pair = 1.f / (float)pairs;
     int4 info = make_int4(0, 0, 0, 0);
     bool more = true;
     const auto take = [&]() {
         if (!ahead) claimed = claim();
         item = __shfl_sync(0xffffffffu, claimed, 0);
         more = item < total && __shfl_sync(0xffffffffu, claimed, 1) == 0;
-        if (more) info = __ldcg(g.gact + 1 + item % per_round / pairs);
+        if (more) {
+            // (this warp's items come in order; below 2^24 a round, so the quotient
+            // is off by one at most)
+            while (item - round_at >= per_round) {
+                round_at += per_round;
+                ++round;
+            }
+            int i = (int)((float)(item - round_at) * per_pair);
+            pair = item - round_at - i * pairs;
+            if (pair < 0) {
+                --i;
+                pair += pairs;
+            } else if (pair >= pairs) {
+                ++i;
+                pair -= pairs;
+            }
+            info = i < GS_ACT ? act[i] : __ldcg(g.gact + 1 + i);
+        }
     };
     if (ahead) {
         claimed = claim();
@@ -597,8 +623,8 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
         while (more) {
             const int now_item = item;
             if (ahead) claimed = claim();     // on its way during what follows
-            r = now_item / per_round;
-            const int p = now_item % pairs, jj = info.x, C = info.z;
+            r = round;
+            const int p = pair, jj = info.x, C = info.z;
             L = info.y;
             vrows = info.w;
             const int nb = block_count(C);
@@ -643,10 +669,7 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
                 const bool quiet = __shfl_sync(0xffffffffu, q >= 0 && q > cI && q > cJ, 0) && nb > 2;
                 if (quiet || (r > 0 && J * GS_BC >= C)) {
                     visit = false;
-                    if (lane == 0) {
-                        st_state(bst + I, tbase + r + 1, cI);
-                        st_state(bst + J, tbase + r + 1, cJ);
-                    }
+                    st_states(bst, I, J, tbase + r + 1, cI, cJ, lane);
                 }
             }
             if (visit) j = jj;
@@ -814,12 +837,9 @@ __device__ __forceinline__ void solver_role(const TwoQGeom& g, const SweepSync& 
         slot_wait(&sl.b_done, par, expired);
         if (lane == 0) {
             mbar_arrive(&sl.b_free);
-            int2* bst = g.gstate + (size_t)j * g.nbmax;
             if (!work) *reinterpret_cast<volatile int*>(qst) = now;
-            __threadfence();
-            st_state(bst + I, now, work ? now : cI);
-            st_state(bst + J, now, work ? now : cJ);
         }
+        st_states(g.gstate + (size_t)j * g.nbmax, I, J, now, work ? now : cI, work ? now : cJ, lane);
         __syncwarp();
     }
     if (expired && lane == 0) atomicExch(sync.error, 1);
@@ -908,9 +928,11 @@ template <int LW, int B, int S, int NG, int NA>
 __global__ void __launch_bounds__((NA + NG + S + 1) * 32, 1)
 gram_sweep_kernel(TwoQGeom g, float tol2, SweepSync sync, int tbase) {
     extern __shared__ __align__(16) float2 gs_sm[];
-    if (__ldcg(&g.gact[0].x) == 0) return;    // no job left to sweep here
+    const int left = __ldcg(&g.gact[0].x);
+    if (left == 0) return;                    // no job left to sweep here
     cf* Xs = gs_sm;
-    Slot<NG>* slots = reinterpret_cast<Slot<NG>*>(Xs + (size_t)B * GS_W * (LW + 2));
+    int4* act = reinterpret_cast<int4*>(Xs + (size_t)B * GS_W * (LW + 2));
+    Slot<NG>* slots = reinterpret_cast<Slot<NG>*>(act + GS_ACT);
     uint64_t* b_read = reinterpret_cast<uint64_t*>(slots + S);       // buffers read out
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < S) {
@@ -927,13 +949,14 @@ gram_sweep_kernel(TwoQGeom g, float tol2, SweepSync sync, int tbase) {
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
+    for (int i = threadIdx.x; i < min(left, GS_ACT); i += blockDim.x) act[i] = __ldcg(g.gact + 1 + i);
     if (B < S && warp == S && lane < B) {
         mbar_init(b_read + lane, NA);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     const int role = (int)(blockDim.x >> 5) - 1 - warp;          // apply warps first
-    if (role == 0) loader<LW, B, S, NG>(g, tol2, sync, tbase, Xs, b_read, slots, lane);
+    if (role == 0) loader<LW, B, S, NG>(g, tol2, sync, tbase, Xs, b_read, act, slots, lane);
     else if (role <= S) solver_role<LW, S, NG>(g, sync, slots[role - 1], lane);
     else if (role <= S + NG) gram_role<LW, S, NG>(sync, Xs, slots, role - 1 - S, lane);
     else apply_role<LW, B, S, NG, NA>(g, sync, Xs, b_read, slots, role - 1 - S - NG, lane);
