@@ -57,6 +57,7 @@
 // parameters twice).
 #include <limits.h>
 
+#include "presort.cuh"
 #include "rot.cuh"
 #include "tc.cuh"
 #include "twoq.cuh"
@@ -578,10 +579,10 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
         return v;
     };
     // Claiming ahead keeps an item waiting behind the present one: only where a
-    // round gives every SM several visits more than it has slots (6.7 an SM, 32
-    // theta of 512 x 512: 22.0 against 23.1 ms a layer; 3.8, 16 of 576 x 576:
-    // 15.7 against 15.3).
-    const bool ahead = per_round > 6 * (int)gridDim.x;
+    // round gives every SM more visits than it has slots (up to 6.5 an SM, 31
+    // theta of 512 x 512: 18.8 ms a layer with it down to 3 an SM, 19.35 down to 6;
+    // 3.8, 16 of 576 x 576: 14.4 ms with it, 14.1 without).
+    const bool ahead = per_round > 4 * (int)gridDim.x;
     int claimed = 0, item = 0;
     int round = 0, round_at = 0, pair = 0;    // the item's round, that round's first item, its pair
     const float per_pair = 1.f / (float)pairs;
@@ -963,17 +964,46 @@ gram_sweep_kernel(TwoQGeom g, float tol2, SweepSync sync, int tbase) {
 }
 
 // The jobs left (not done, and not the tensor-core sweeps' in a mixed call), in
-// order, into gact; the sweep's counters cleared.  One block.
-constexpr int GS_BEGIN_T = 512;
+// order, into gact; the sweep's counters cleared.  One block -- or, where the
+// columns are sorted, a block a job, which ends the job's sweep and sorts it, and
+// the last block to finish goes on to the list (a kernel of its own for the sort
+// cost a launch, ~5 us, a sweep).
+constexpr int GS_BEGIN_T = PRESORT_T;
 
 __global__ void __launch_bounds__(GS_BEGIN_T)
 gram_begin_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs, SweepSync sync,
                   GramBegin b) {
     __shared__ int s_warp[GS_BEGIN_T / 32];
-    __shared__ int s_nb;
+    __shared__ int s_nb, s_flag;
+    extern __shared__ __align__(16) float s_sort[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (b.sort_cols) {
+        const int j = blockIdx.x;
+        if (tid == 0) {
+            bool open = !g.done[j];
+            if (open && b.end_sweep) {
+                if (!(g.offmax[j] > b.tol2)) {
+                    g.done[j] = 1;
+                    open = false;
+                }
+                g.offmax[j] = 0.f;
+            }
+            s_flag = open ? 1 : 0;
+        }
+        __syncthreads();
+        if (s_flag) presort_job(jobs[j], g, j, s_sort, GS_BC, b.tpre);
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            s_flag = atomicAdd(g.counter + 7, 1) == njobs - 1;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!s_flag) return;
+    }
     if (tid == 0) {
         s_nb = 0;
+        g.counter[7] = 0;
         g.counter[0] = 0;
         *sync.next_item = 0;
         if (g.tc_mode) g.counter[4] = g.counter[5] = 0;
@@ -987,8 +1017,8 @@ gram_begin_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int njobs, Sw
         const int j = j0 + tid;
         bool live = false;
         int4 e = make_int4(j, 0, 0, 0);
-        bool open = j < njobs && !g.done[j];
-        if (open && b.end_sweep) {
+        bool open = j < njobs && !__ldcg(g.done + j);
+        if (open && b.end_sweep && !b.sort_cols) {
             if (!(g.offmax[j] > b.tol2)) {
                 g.done[j] = 1;
                 open = false;
@@ -1064,7 +1094,8 @@ int launch(int njobs, int rounds, int pairs, const TwoQGeom& g, float tol2, cons
 
 int gram_begin_launch(const mps_2q_job* jobs, int njobs, const TwoQGeom& g, const SweepSync& sync,
                       const GramBegin& b, cudaStream_t s) {
-    gram_begin_kernel<<<1, GS_BEGIN_T, 0, s>>>(jobs, g, njobs, sync, b);
+    gram_begin_kernel<<<b.sort_cols ? njobs : 1, GS_BEGIN_T, presort_smem(b.sort_cols), s>>>(
+        jobs, g, njobs, sync, b);
     MPS_LAUNCH_CHECK("gram_begin_kernel");
     return MPS_OK;
 }

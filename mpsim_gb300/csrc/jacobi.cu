@@ -52,6 +52,7 @@
 #include <string>
 
 #include "gemm.cuh"
+#include "presort.cuh"
 #include "rot.cuh"
 #include "twoq.cuh"
 
@@ -723,73 +724,12 @@ __global__ void count_simt_jobs_kernel(const mps_2q_job* __restrict__ jobs, int 
 // left in cnrm (theta_norm_kernel's before the first sweep) and rewrites the
 // job's column map.  Converged jobs keep theirs, and so do the tensor-core
 // jobs of a mixed call (see below).
-constexpr int PRESORT_T = 512;
-
 __global__ void __launch_bounds__(PRESORT_T)
-presort_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int npow2, int bc, int tpre) {
-    extern __shared__ float2 sm1[];
-    float* key = reinterpret_cast<float*>(sm1);
-    int* idx = reinterpret_cast<int*>(key + npow2);
+presort_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int bc, int tpre) {
+    extern __shared__ __align__(16) float sm1[];
     const int j = blockIdx.x;
     if (__ldg(g.done + j)) return;
-    const int m = jobs[j].chi_l * g.d, n = jobs[j].chi_r * g.d;
-    const int C = min(m, n);
-    if (C < 2) return;
-    // The tensor-core sweeps keep their columns in place: measured, their jobs
-    // converge about a sweep sooner unsorted (the LQ factor's own column order,
-    // and blocks that keep their columns keep their visits skippable), while
-    // the SIMT sweeps gain from the sort.
-    if (g.tc_mode && tc_job(m, n, jobs[j].keep_left_canonical)) return;
-    const int tid = threadIdx.x;
-    const float* cn = g.cnrm + (size_t)j * g.cslot;
-    for (int i = tid; i < npow2; i += PRESORT_T) {
-        float k = -1.f;
-        if (i < C) {
-            k = cn[i];
-            if (!(k == k)) k = 0.f;                  // NaN sorts as zero
-        }
-        key[i] = k;
-        idx[i] = i;
-    }
-    __syncthreads();
-    for (int size = 2; size <= npow2; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = tid; i < npow2; i += PRESORT_T) {
-                const int pj = i ^ stride;
-                if (pj > i) {
-                    const bool desc = (i & size) == 0;
-                    const float ki = key[i], kj = key[pj];
-                    const int ii = idx[i], ij = idx[pj];
-                    const bool i_first = (ki > kj) || (ki == kj && ii < ij);
-                    if (i_first != desc) {
-                        key[i] = kj; key[pj] = ki;
-                        idx[i] = ij; idx[pj] = ii;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    if (g.vstamp) {
-        // a block whose set of columns changes counts as changed (its pairs
-        // are not the ones last checked); moves inside a block do not, except
-        // for the Gram sweeps, whose block products go by position
-        int* oldpos = reinterpret_cast<int*>(key);     // the keys are no longer needed
-        for (int i = tid; i < C; i += PRESORT_T) oldpos[__ldcg(g.cmap + (size_t)j * g.cslot + i)] = i;
-        __syncthreads();
-        int* vst = g.vstamp + (size_t)j * g.nbmax;
-        int2* bst = g.gstate + (size_t)j * g.nbmax;
-        for (int c = tid; c < C; c += PRESORT_T) {
-            const int ob = oldpos[idx[c]] / bc, nb = c / bc;
-            if (g.gstate) {
-                if (oldpos[idx[c]] != c) bst[ob].y = bst[nb].y = tpre;
-            } else if (ob != nb) {
-                vst[ob] = tpre;
-                vst[nb] = tpre;
-            }
-        }
-    }
-    for (int i = tid; i < C; i += PRESORT_T) g.cmap[(size_t)j * g.cslot + i] = idx[i];
+    presort_job(jobs[j], g, j, sm1, bc, tpre);
 }
 
 // ---------------------------------------------------------------------------
@@ -1562,6 +1502,7 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
     int npow2 = 1;
     while (npow2 < lo.cslot) npow2 <<= 1;
     const size_t sort_smem = (size_t)npow2 * (sizeof(float) + sizeof(int));
+    const int sort_cols = cmax > 2 * bc ? lo.cslot : 0;      // (one visit covers fewer)
     int sweeps = 0;
     bool converged = false;
     if (cmax >= 2) {
@@ -1576,15 +1517,12 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
         const bool piped = gram && !mixed && !capturing;
         for (sweeps = 1; piped; ++sweeps) {
             const int seq = ++t_seq;
-            rc = gram_begin_launch(jobs, njobs, g, sync, GramBegin{sweeps > 1, sweeps == 1, tol2,
-                                                                   t_pinned, seq}, s);
+            rc = gram_begin_launch(jobs, njobs, g, sync,
+                                   GramBegin{sweeps > 1, sweeps == 1, tol2, t_pinned, seq,
+                                             sweeps <= max_sweeps ? sort_cols : 0,
+                                             sweeps * tbase_stride}, s);
             if (rc) return rc;
             if (sweeps <= max_sweeps) {
-                if (cmax > 2 * bc) {
-                    presort_kernel<<<njobs, PRESORT_T, sort_smem, s>>>(jobs, g, npow2, bc,
-                                                                       sweeps * tbase_stride);
-                    MPS_LAUNCH_CHECK("presort_kernel");
-                }
                 rc = gram_sweep_launch(njobs, rounds, pairs, g, asked, sync, sweeps * tbase_stride, s);
                 if (rc) return rc;
             }
@@ -1603,16 +1541,17 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
             }
         }
         for (sweeps = piped ? sweeps : 1; !piped && sweeps <= max_sweeps; ++sweeps) {
-            if (cmax > 2 * bc) {
-                presort_kernel<<<njobs, PRESORT_T, sort_smem, s>>>(jobs, g, npow2, bc,
-                                                                   sweeps * tbase_stride);
-                MPS_LAUNCH_CHECK("presort_kernel");
-            }
             if (gram) {
-                rc = gram_begin_launch(jobs, njobs, g, sync, GramBegin{false, !mixed, tol2, nullptr, 0},
-                                       s);
+                rc = gram_begin_launch(jobs, njobs, g, sync,
+                                       GramBegin{false, !mixed, tol2, nullptr, 0, sort_cols,
+                                                 sweeps * tbase_stride}, s);
                 if (rc) return rc;
             } else {
+                if (sort_cols) {
+                    presort_kernel<<<njobs, PRESORT_T, presort_smem(lo.cslot), s>>>(
+                        jobs, g, bc, sweeps * tbase_stride);
+                    MPS_LAUNCH_CHECK("presort_kernel");
+                }
                 MPS_CUDA_CHECK(cudaMemsetAsync(g.counter, 0, sizeof(int), s));
                 if (mixed) MPS_CUDA_CHECK(cudaMemsetAsync(g.counter + 4, 0, 2 * sizeof(int), s));
                 MPS_CUDA_CHECK(cudaMemsetAsync(sync.next_item, 0, (mixed ? 1 : 2) * sizeof(int), s));
@@ -1878,7 +1817,7 @@ extern "C" int mps_apply_2q_batch_noalloc(void* stream, const mps_2q_job* jobs, 
         for (sweeps = 1; sweeps <= max_sweeps; ++sweeps) {
             MPS_CUDA_CHECK(cudaMemsetAsync(g.counter, 0, sizeof(int), s));
             if (cmax > 2 * bc) {
-                presort_kernel<<<njobs, PRESORT_T, sort_smem, s>>>(jobs, g, npow2, bc, 0);
+                presort_kernel<<<njobs, PRESORT_T, presort_smem(lo.cslot), s>>>(jobs, g, bc, 0);
                 MPS_LAUNCH_CHECK("presort_kernel");
             }
             for (int r = 0; r < rounds; ++r) {

@@ -144,12 +144,14 @@ constexpr int kGramBlock = 8;
 // counter[0] (and [4], [5] of a mixed call) and the item counter; as asked it
 // first ends the sweep before (jobs without a pair over the tolerance are
 // done), clears the error word, and writes (jobs left, NaN count, error word,
-// seq) to a record in pinned host memory.
+// seq) to a record in pinned host memory.  With sort_cols (the slots' columns) it
+// also sorts the columns of the jobs left (presort_job, at time tpre).
 struct GramBegin {
     bool end_sweep, clear_error;
     float tol2;
     int* record;
     int seq;
+    int sort_cols, tpre;
 };
 int gram_begin_launch(const mps_2q_job* jobs, int njobs, const TwoQGeom& g, const SweepSync& sync,
                       const GramBegin& b, cudaStream_t s);
