@@ -56,3 +56,18 @@ def test_buffers_fewer_than_slots(built_lib, cuda, chil, chir, lc):
     assert rc == 0, _native.last_error()
     for spec, out in zip(specs, res):
         check_job(spec, out, 2)
+
+
+@pytest.mark.parametrize("n", [20, 70, 130])
+def test_infinite_entry_is_reported(built_lib, cuda, n):
+    """The column sort keeps a valid order when norms overflow; the call ends with
+    its error and the next one is right."""
+    rng = np.random.default_rng(n)
+    a, b, g = make_job_inputs(rng, n, n, n, 2, scale=1.0 / n)
+    bad = a.copy()
+    bad[n // 2, 1, n // 3] = np.inf
+    rc, _, _ = run_batch(built_lib, cuda, [(bad, b, g, n, True)])
+    assert rc == _native.MPS_ERR_NONFINITE
+    rc, res, _ = run_batch(built_lib, cuda, [(a, b, g, n, True)])
+    assert rc == 0, _native.last_error()
+    check_job((a, b, g, n, True), res[0], 2)
