@@ -48,12 +48,11 @@ def gate_flops(m, n, chim, d):
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of a chi=256
-# two-qudit call of 32 jobs, from one ncu capture per kernel (three launches
-# each, caches left warm) scaled by the launch counts of one call: per sweep
-# of the plain sweep kernel, and for the rest of the call (merge, LQ,
-# post-GEMMs, sorts).  A call's traffic is sweeps x the first + the second.
-SWEEP_TRAFFIC_BYTES = 1.12e9
-CALL_OTHER_TRAFFIC_BYTES = 1.16e9
+# two-qudit call of 32 jobs, from one ncu capture of a call's launches (caches
+# left warm): per sweep of the plain sweep kernel, and for the rest of the call
+# (merge, LQ, post-GEMMs, sorts).  A call's traffic is sweeps x the first + the second.
+SWEEP_TRAFFIC_BYTES = 1.03e9
+CALL_OTHER_TRAFFIC_BYTES = 0.91e9
 
 
 def replica_instance(rank: int) -> int:

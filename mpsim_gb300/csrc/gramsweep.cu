@@ -43,7 +43,7 @@
 // own: once the apply warps hold a visit's rows in registers its buffer takes the
 // next visit's columns, while the rotations and the write-back go on.
 //
-// Measured (GB300): 32 theta of 512 x 512, mean sweep 1.21 ms against 1.76 of the
+// Measured (GB300): 31 theta of 512 x 512, mean sweep 1.16 ms against 1.76 of the
 // column-by-column kernel (57% of the issue slots busy at four warps a scheduler;
 // L2 26%).  Buffers apart from the slots, against a slot that kept its columns to
 // the end: layers of 40 sites chi=420 (one buffer of 1024 rows) 58.3 -> 51.7 ms, of
