@@ -74,7 +74,7 @@ typedef struct {
     int32_t block_cols;    /* out: columns per block the kernel used       */
     int32_t sweeps_out;    /* out: sweeps taken by the slowest job         */
     int32_t wait_limit;    /* max polls of a round-dependency wait inside a
-                              sweep (default 1<<22, ~0.3 s); on expiry the
+                              sweep (default 1<<22, 1-3 s); on expiry the
                               call returns MPS_ERR_TIMEOUT                 */
     int32_t stall_test;    /* test hook: nonzero makes one wait target a
                               round that never completes, so the wait must

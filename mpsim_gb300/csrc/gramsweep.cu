@@ -74,7 +74,6 @@ constexpr int GS_NBLK = GS_BC * (GS_BC - 1) / 2;   // 2 x 2 blocks off the diago
 constexpr int GS_LEAD = 3;                   // step the solver has taken when a warp starts
                                              // (1 where each slot has its own buffer)
 constexpr int GS_ACT = 256;                  // jobs left that a CTA keeps in shared memory
-constexpr int GS_TRIES = 1 << 20;            // suspended tries of a slot wait
 constexpr unsigned GS_SUSPEND_NS = 1000;
 constexpr float kInnerTol2 = 0.25f;
 static_assert(GS_BC == 8 && GS_NBLK <= 32, "one solver warp, one 2 x 2 block a lane");
@@ -476,13 +475,13 @@ __device__ __forceinline__ void st_states(int2* bst, int I, int J, int t, int cI
     }
 }
 
-// Waits for a barrier's phase; gives up for good after GS_TRIES suspended tries
-// (the call then reports an expired wait).
-__device__ __forceinline__ void slot_wait(uint64_t* bar, unsigned parity, bool& expired) {
+// Waits for a barrier's phase; gives up for good after limit suspended tries
+// (SweepSync::slot_limit; the call then reports an expired wait).
+__device__ __forceinline__ void slot_wait(uint64_t* bar, unsigned parity, int limit, bool& expired) {
     if (expired) return;
     int tries = 0;
     while (!mbar_try_wait(bar, parity, GS_SUSPEND_NS)) {
-        if (++tries > GS_TRIES) {
+        if (++tries > limit) {
             expired = true;
             break;
         }
@@ -496,11 +495,11 @@ __device__ __forceinline__ void slot_wait(uint64_t* bar, unsigned parity, bool& 
 // steps are waited for two at a time, unless the last one is there already.
 template <int NG>
 __device__ __forceinline__ void apply_ring(Row2 (&y)[GS_W], Slot<NG>& sm, unsigned parity,
-                                           bool& expired) {
+                                           int limit, bool& expired) {
     const bool ready = __all_sync(0xffffffffu, mbar_test_wait(sm.b_ring + GS_BC - 1, parity));
 #pragma unroll 1
     for (int s = 0; s < GS_BC; s += 2) {
-        if (!ready) slot_wait(sm.b_ring + s + 1, parity, expired);
+        if (!ready) slot_wait(sm.b_ring + s + 1, parity, limit, expired);
         const uint2 m = *reinterpret_cast<const uint2*>(sm.mask + s);
         if (m.x) {
 #pragma unroll
@@ -526,10 +525,10 @@ __device__ __forceinline__ void apply_ring(Row2 (&y)[GS_W], Slot<NG>& sm, unsign
 // steps every column is back at its own.
 template <int NG>
 __device__ __forceinline__ void apply_full(Row2 (&y)[GS_W], Slot<NG>& sm, unsigned parity,
-                                           bool& expired) {
+                                           int limit, bool& expired) {
 #pragma unroll 1
     for (int s = 0; s < GS_FULL; ++s) {
-        slot_wait(sm.b_circle + s, parity, expired);
+        slot_wait(sm.b_circle + s, parity, limit, expired);
         if (sm.mask[s] != 0) {
 #pragma unroll
             for (int k = 0; k < GS_BC; ++k) rotate2(y[k], y[GS_FULL - k], sm.prm[s * GS_BC + k]);
@@ -679,7 +678,7 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
             if (visit) break;
         }
         // ---- into the slot ---------------------------------------------------
-        if (t.use > 0) slot_wait(&sl.b_free, t.parity() ^ 1u, expired);
+        if (t.use > 0) slot_wait(&sl.b_free, t.parity() ^ 1u, sync.slot_limit, expired);
         if (j < 0) {
             --left;
             if (lane == 0) {
@@ -689,7 +688,7 @@ __device__ __forceinline__ void loader(const TwoQGeom& g, float tol2, const Swee
                 mbar_arrive(&sl.b_full);
             }
         } else {
-            if (B < S && tb.use > 0) slot_wait(b_read + tb.slot, tb.parity() ^ 1u, expired);
+            if (B < S && tb.use > 0) slot_wait(b_read + tb.slot, tb.parity() ^ 1u, sync.slot_limit, expired);
             const uint32_t bytes = (uint32_t)((L + 63) >> 6) * 64u * (uint32_t)sizeof(cf);
             if (lane < GS_W) sl.col[lane] = col;
             if (lane == 0) {
@@ -734,7 +733,7 @@ __device__ __forceinline__ void gram_role(const SweepSync& sync, const cf* Xs, S
     bool expired = false;
     for (;; t.next()) {
         Slot<NG>& sl = slots[t.slot];
-        slot_wait(&sl.b_full, t.parity(), expired);
+        slot_wait(&sl.b_full, t.parity(), sync.slot_limit, expired);
         if (sl.job < 0 || expired) break;
         const int L = sl.L, np = sl.full ? 3 : 1;
         const cf* X = Xs + (size_t)sl.buf * GS_W * XST;
@@ -754,7 +753,7 @@ __device__ __forceinline__ void solver_role(const TwoQGeom& g, const SweepSync& 
                                             int lane) {
     bool expired = false;
     for (unsigned par = 0u;; par ^= 1u) {
-        slot_wait(&sl.b_info, par, expired);
+        slot_wait(&sl.b_info, par, sync.slot_limit, expired);
         const int j = sl.job;
         if (j < 0 || expired) {
             if (lane == 0) {
@@ -782,7 +781,7 @@ __device__ __forceinline__ void solver_role(const TwoQGeom& g, const SweepSync& 
                 }
             }
         }
-        slot_wait(&sl.b_gram, par, expired);
+        slot_wait(&sl.b_gram, par, sync.slot_limit, expired);
         // the squared norms (lane l: column l & 15), then every product against
         // them as it is summed
         float nrm = 0.f;
@@ -835,7 +834,7 @@ __device__ __forceinline__ void solver_role(const TwoQGeom& g, const SweepSync& 
         const int now = sl.time, cI = sl.changedI, cJ = sl.changedJ;
         int* qst = sl.qst;
         __syncwarp();
-        slot_wait(&sl.b_done, par, expired);
+        slot_wait(&sl.b_done, par, sync.slot_limit, expired);
         if (lane == 0) {
             mbar_arrive(&sl.b_free);
             if (!work) *reinterpret_cast<volatile int*>(qst) = now;
@@ -856,7 +855,7 @@ __device__ __forceinline__ void apply_role(const TwoQGeom& g, const SweepSync& s
     int first = aw;                           // this warp's first task of the visit
     for (;; t.next()) {
         Slot<NG>& sl = slots[t.slot];
-        slot_wait(&sl.b_work, t.parity(), expired);
+        slot_wait(&sl.b_work, t.parity(), sync.slot_limit, expired);
         const int j = sl.job;
         if (j < 0 || expired) break;
         bool reading = B < S;                 // the visit's column buffer
@@ -875,7 +874,7 @@ __device__ __forceinline__ void apply_role(const TwoQGeom& g, const SweepSync& s
             // steps as they come.  (Where a buffer waits for it, the warp takes
             // the columns first.)
             uint64_t* start = full ? sl.b_circle + GS_FULL / 2 : sl.b_ring + (B < S ? GS_LEAD : 1);
-            if (B == S && q < np) slot_wait(start, par, expired);
+            if (B == S && q < np) slot_wait(start, par, sync.slot_limit, expired);
 #pragma unroll 1
             for (; q < np; q += NA) {
                 const bool in_x = q < xp;
@@ -901,9 +900,9 @@ __device__ __forceinline__ void apply_role(const TwoQGeom& g, const SweepSync& s
                     lane0_arrive(b_read + sl.buf, lane);
                     reading = false;
                 }
-                if (B < S && q == first) slot_wait(start, par, expired);
-                if (full) apply_full(y, sl, par, expired);
-                else apply_ring(y, sl, par, expired);
+                if (B < S && q == first) slot_wait(start, par, sync.slot_limit, expired);
+                if (full) apply_full(y, sl, par, sync.slot_limit, expired);
+                else apply_ring(y, sl, par, sync.slot_limit, expired);
 #pragma unroll
                 for (int c = 0; c < GS_W; ++c) rescale2(y[c], sl.scale[c]);
                 if (live) {

@@ -1454,6 +1454,9 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
     sync.block_round = sync.next_item + 2;
     sync.nbmax = lo.nbmax;
     sync.wait_limit = (params && params->wait_limit > 0) ? params->wait_limit : (1 << 22);
+    // (a suspended try lasts longer than 2.2 us and a poll 0.3-0.7 us, so that the
+    // loader's own wait ends first)
+    sync.slot_limit = max(sync.wait_limit, 1 << 20);
     sync.stall_test = params ? params->stall_test : 0;
     // padding rows and columns of X must be zero
     MPS_CUDA_CHECK(cudaMemsetAsync(g.X, 0, lo.off_V - lo.off_X, s));

@@ -71,6 +71,9 @@ struct SweepSync {
     int* block_round; // [njobs][nbmax]: last round each block finished (-1)
     int nbmax;
     int wait_limit;
+    // suspended tries of the Gram sweeps' waits inside a CTA: what they wait for may
+    // itself be a wait of wait_limit polls
+    int slot_limit;
     int stall_test;
 };
 
