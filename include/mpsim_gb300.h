@@ -253,7 +253,11 @@ int mps_tc_error(int* flag_out);
 int mps_tc_profile(unsigned long long* out10, int reset);
 
 /* Workspace for mps_site_marginals: two environments a direction and, for
- * each direction, a (chi_l, d, chi_r) product of every site. */
+ * each direction, a (chi_l, d, chi_r) product of every site -- twice the state
+ * -- up to 16 GiB; beyond, the least that the call takes (with which it forms a
+ * product a site more): the left environments, two right ones and the products
+ * of the largest site, (sum_i chi_i^2 (i < n) + 2 (1 + d) max_chi^2) complex64,
+ * n d floats and 1024 bytes, rounded up to 256. */
 size_t mps_marginals_workspace_bytes(const int* chis, int n, int d);
 
 /* The diagonal of every single-site reduced density matrix,
