@@ -202,7 +202,8 @@ int mps_wavefunction(void* stream, const mps_c64* const* sites,
  * 2 * nbits * d * max_chi complex64, or better
  * mps_amplitudes_workspace_bytes(), which leaves room to group the bitstrings
  * by digit at every site (each then multiplies one of the site's d matrices
- * instead of all). */
+ * instead of all): 2 * nbits * max_chi complex64 and up to 256 MiB, or the
+ * former where that is more. */
 size_t mps_amplitudes_workspace_bytes(int nbits, int max_chi, int n, int d);
 int mps_amplitudes(void* stream, const mps_c64* const* sites, const int* chis,
                    int n, int d, const int8_t* bits_dev, int nbits,

@@ -684,11 +684,23 @@ size_t amplitude_counts(int nbits, int n, int d) {
     const int chunks = group_chunks(nbits);
     return chunks > 1 ? (size_t)n * chunks * (min(d, kDigits) + 1) : 0;
 }
-size_t amplitude_bytes(int nbits, int maxchi, int n, int d) {
+// Lists of n sites.
+size_t amplitude_lists(int nbits, int maxchi, int n, int d) {
     const int tile = amplitude_tile(nbits, maxchi, d);
     const size_t tiles = (size_t)amplitude_tiles(nbits, d, tile);
+    return ((size_t)n * tiles * (tile + 1) + amplitude_counts(nbits, n, d)) * sizeof(int);
+}
+// Sites whose lists are made together: all of them, if the lists stay within 256 MiB or
+// within what a product of every digit would take (4 10^6 bitstrings of 1000 sites
+// would be 16 GB); else as many as do, and the lists are made again for the next ones.
+int amplitude_group_sites(int nbits, int maxchi, int n, int d) {
+    const size_t room = max((size_t)256 << 20, (size_t)nbits * d * maxchi * sizeof(cf));
+    const size_t sites = room / amplitude_lists(nbits, maxchi, 1, d);
+    return sites < 1 ? 1 : (int)min(sites, (size_t)n);
+}
+size_t amplitude_bytes(int nbits, int maxchi, int n, int d) {
     return 2 * (size_t)nbits * maxchi * sizeof(cf) +
-           ((size_t)n * tiles * (tile + 1) + amplitude_counts(nbits, n, d)) * sizeof(int);
+           amplitude_lists(nbits, maxchi, amplitude_group_sites(nbits, maxchi, n, d), d);
 }
 
 }  // namespace
@@ -716,21 +728,23 @@ extern "C" int mps_amplitudes(void* stream, const mps_c64* const* sites, const i
         amplitude_tiles(nbits, d, tile) <= 65535) {
         cf* ge[2] = {static_cast<cf*>(workspace), static_cast<cf*>(workspace) + env_sz};
         const int tiles = amplitude_tiles(nbits, d, tile);
+        const int group = amplitude_group_sites(nbits, maxchi, n, d), nd = min(d, kDigits);
         int* rows = reinterpret_cast<int*>(ge[1] + env_sz);
-        int* digit = rows + (size_t)n * tiles * tile;
-        int* counts = digit + (size_t)n * tiles;
-        const int nd = min(d, kDigits);
-        const dim3 groups(n, group_chunks(nbits));
+        int* digit = rows + (size_t)group * tiles * tile;
+        int* counts = digit + (size_t)group * tiles;
         fill_one_kernel<<<grid_for(nbits), 256, 0, s>>>(ge[0], nbits);
         MPS_LAUNCH_CHECK("fill_one_kernel");
-        if (groups.y > 1) {
-            count_digits_kernel<<<groups, kGroupT, 0, s>>>(bits_dev, nbits, n, nd, counts);
-            MPS_LAUNCH_CHECK("count_digits_kernel");
-        }
-        group_bits_kernel<<<groups, kGroupT, 0, s>>>(bits_dev, nbits, n, nd, tile, tiles, counts, rows,
-                                                     digit);
-        MPS_LAUNCH_CHECK("group_bits_kernel");
         for (int i = 0, at = 0; i < n; ++i, at ^= 1) {
+            if (i % group == 0) {
+                const dim3 grid(min(group, n - i), group_chunks(nbits));
+                if (grid.y > 1) {
+                    count_digits_kernel<<<grid, kGroupT, 0, s>>>(bits_dev + i, nbits, n, nd, counts);
+                    MPS_LAUNCH_CHECK("count_digits_kernel");
+                }
+                group_bits_kernel<<<grid, kGroupT, 0, s>>>(bits_dev + i, nbits, n, nd, tile, tiles,
+                                                           counts, rows, digit);
+                MPS_LAUNCH_CHECK("group_bits_kernel");
+            }
             const int cl = chis[i], cr = chis[i + 1];
             if (cr == 0) continue;
             cf* dst = (i == n - 1) ? reinterpret_cast<cf*>(out_dev) : ge[at ^ 1];
@@ -738,7 +752,8 @@ extern "C" int mps_amplitudes(void* stream, const mps_c64* const* sites, const i
             gl.p[0] = GemmArgs{tiles * tile, cr, cl, ge[at], cl, 1, 0,
                                reinterpret_cast<const cf*>(sites[i]), (long long)d * cr, 1, 0,
                                dst, cr, 1};
-            gl.ga = GemmGather{rows + (size_t)i * tiles * tile, digit + (size_t)i * tiles, cr, nd};
+            gl.ga = GemmGather{rows + (size_t)(i % group) * tiles * tile,
+                               digit + (size_t)(i % group) * tiles, cr, nd};
             const dim3 grid((cr + tile - 1) / tile, tiles);
             const int rc = tile == 32
                                ? launch_gather(cgemm_kernel<32, 32, 4, false, true>, 32, grid, s, gl)

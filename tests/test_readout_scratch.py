@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from mpsim_gb300 import _native
+from mpsim_gb300 import MPS, _native
 from test_gpu_readout_tiles import CHAINS, EPS, _chain
 
 GUARD = 4096
@@ -30,6 +30,31 @@ def test_marginal_scratch_is_bounded(built_lib, n, chi, d):
     chis = [1] + [chi] * (n - 1) + [1]
     need = built_lib.mps_marginals_workspace_bytes(_ints(chis), n, d)
     assert 0 < need <= max(16 << 30, _lean_marginals(chis, d))
+
+
+@pytest.mark.parametrize("nbits,chi,n,d", [(4096, 256, 64, 2), (1, 1, 1, 2), (4 * 10 ** 6, 1, 1000, 2),
+                                           (10 ** 6, 16, 5000, 3), (10 ** 6, 256, 64, 2)])
+def test_amplitude_scratch_is_bounded(built_lib, nbits, chi, n, d):
+    """Two environments and 256 MiB, or a product of every digit, if that is more; it
+    does not grow with the chain."""
+    need = built_lib.mps_amplitudes_workspace_bytes(nbits, chi, n, d)
+    env = nbits * chi * 8
+    assert (d + 2) * env <= need <= max((d + 2) * env, 2 * env + (256 << 20))
+
+
+@pytest.mark.gpu
+def test_amplitudes_of_a_chain_listed_in_parts(cuda):
+    """More sites than lists fit in 256 MiB (470 of them here), the last part shorter.  Sites
+    of bond 1 with entries of modulus 1; a complex product is off by 2 sqrt(2) 2^-24."""
+    rng = np.random.default_rng(2)
+    n, count = 500, 140000
+    phase = np.exp(2j * np.pi * rng.random((n, 1, 2, 1))).astype(np.complex64)
+    bits = rng.integers(0, 2, (count, n), dtype=np.int8)
+    ref = np.ones(count, np.complex128)
+    for i in range(n):
+        ref *= phase[i, 0, bits[:, i], 0].astype(np.complex128)
+    mps = MPS.from_sites([torch.from_numpy(t).to(cuda) for t in phase], 2)
+    assert np.max(np.abs(mps.amplitudes(bits) - ref)) <= n * 2 * np.sqrt(2) * EPS * np.max(np.abs(ref))
 
 
 @pytest.mark.gpu
