@@ -1431,8 +1431,9 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
         if (params->max_sweeps > 0) max_sweeps = params->max_sweeps;
         tol = params->tol;
     }
-    // the kernels compare squared cosines (asked: the caller's tolerance, if any)
-    const float asked = tol > 0.f ? tol * tol : 0.f;
+    // the kernels compare squared cosines (asked: the caller's tolerance, if any; one
+    // whose square underflows is still asked for)
+    const float asked = tol > 0.f ? fmaxf(tol * tol, FLT_MIN) : 0.f;
     const float tol2 = asked > 0.f ? asked : default_tol2(lo.lslot);
     const bool mixed = params && params->precision == MPS_PRECISION_MIXED;
     if (params && params->precision != MPS_PRECISION_PLAIN && !mixed)
