@@ -6,8 +6,8 @@ The choices it makes per call (fields of ``mps_svd_params``):
   factor (the LQ factorisation costs panels on a few SMs; the sweeps it saves
   depend on the shape);
 * ``block_request`` -- the plain sweeps' block width for 512 / 576-row slots; the
-  library takes 0, 8 and 16 and uses 8-column blocks for each, so today its
-  candidates measure alike;
+  library takes 0, 8 and 16 and uses 8-column blocks for each, so a table may hold
+  any of them and ``tune()`` measures 0 only;
 * ``precision``     -- for ``MPS(precision="auto")``: the plain FP32 sweeps or
   the tensor-core block sweeps, whichever is faster for that shape and batch.
 
@@ -17,7 +17,7 @@ correctness guard (singular values equal to the default configuration's
 within 1e-4 s_0), and writes the winners to a JSON table; ``lookup()`` reads
 it.  The committed table ``tuning/gb300.json`` was measured on a GB300 with
 ``python -m mpsim_gb300.autotune``; shapes missing from it take the defaults.
-Batch sizes are bucketed (<= 8, <= 64, more): a layer of one 64-qubit circuit
+Batch sizes are bucketed (``BUCKETS``): a layer of one 64-qubit circuit
 is 32 jobs, a batched layer of many circuits thousands.
 """
 
@@ -84,7 +84,8 @@ def lookup(m: int, n: int, d: int, njobs: int, table: Optional[Dict] = None) -> 
 
 
 def candidates(m: int, n: int, lc: bool = True):
-    """(precision, lq_off, block_request) triples valid for this shape."""
+    """(precision, lq_off, block_request) triples valid for this shape (those that
+    differ in block_request alone run the same kernel)."""
     L = max(m, n)
     out = []
     for lq_off in (0, 1):
@@ -161,6 +162,8 @@ def tune(shapes, njobs_list=TUNE_BATCHES, reps: int = 3, device=None, log=print)
             ref_ms, ref = _time(lib, keep, S, nj, m, n, d, ("plain", 0, 0), reps, ws)
             best, best_ms, res = ("plain", 0, 0), ref_ms, {}
             for cand in candidates(m, n):
+                if cand[2]:
+                    continue                  # the same kernel as block_request 0
                 ms, sv = (ref_ms, ref) if cand == ("plain", 0, 0) else \
                     _time(lib, keep, S, nj, m, n, d, cand, reps, ws)
                 if ms is None:
