@@ -42,6 +42,10 @@ TABLE_PATH = os.path.join(HERE, "tuning", "gb300.json")
 # a bucket takes the mixed form only where it wins for every batch it covers.
 BUCKETS = (8, 16, 32, 64, 128, 256, 1 << 30)
 TUNE_BATCHES = (1,) + tuple(b + 1 for b in BUCKETS[:-1])
+# A form with or without the LQ start replaces the other only if it is faster by more
+# than this (two tunings of one library differ by up to 2% in the small entries);
+# plain and mixed are taken as measured.
+NOISE = 0.02
 DEFAULT = {"lq_off": 0, "block_request": 0, "precision": "plain"}
 
 _table = None
@@ -170,7 +174,7 @@ def tune(shapes, njobs_list=TUNE_BATCHES, reps: int = 3, device=None, log=print)
                     continue
                 ok = np.all(np.abs(sv - ref) <= 1e-4 * ref[:, :1] + 1e-30)
                 res["/".join(map(str, cand))] = round(ms, 4) if ok else None
-                if ok and ms < best_ms:
+                if ok and ms < best_ms * (1.0 - NOISE if cand[0] == best[0] else 1.0):
                     best, best_ms = cand, ms
             k = key(m, n, d, nj)
             out[k] = {"precision": best[0], "lq_off": best[1], "block_request": best[2],
