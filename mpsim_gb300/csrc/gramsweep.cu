@@ -44,8 +44,8 @@
 // next visit's columns, while the rotations and the write-back go on.
 //
 // Measured (GB300): 31 theta of 512 x 512, mean sweep 1.16 ms against 1.76 of the
-// column-by-column kernel (57% of the issue slots busy at four warps a scheduler;
-// L2 26%).  Buffers apart from the slots, against a slot that kept its columns to
+// column-by-column kernel (59% of the issue slots busy at four warps a scheduler;
+// L2 27%).  Buffers apart from the slots, against a slot that kept its columns to
 // the end: layers of 40 sites chi=420 (one buffer of 1024 rows) 58.3 -> 51.7 ms, of
 // 32 qutrits chi=192 14.75 -> 14.3, of 64 sites chi=256 19.8 -> 19.4; slots of up to
 // 256 rows have a buffer each (sharing them measured 1-3% slower).  24

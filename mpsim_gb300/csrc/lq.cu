@@ -89,7 +89,9 @@ __device__ __forceinline__ void warp_sum4(float& v0, float& v1, float& v2, float
 // for a row above it is (V^H V)[r][i] up to conj(inv_r) inv_i, which T needs.  The
 // warp of the next pivot row computes its scalars, that of the last one T's column.
 // Mean panel of a 512-column job: 38 us (before, with the rows in shared memory, a
-// warp a row, and T afterwards: 94 us).
+// warp a row, and T afterwards: 94 us).  Beyond 512 columns a part of the rows spills
+// (60 bytes a thread in the kernel for 640, 444 in that for 768); it is still ahead: calls of
+// 16 jobs of 768 columns 52 ms with the factorised start, 57 without it, 104 with it before.
 template <int NT>
 __global__ void __launch_bounds__(LQ_T, 1)
 lq_panel_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g, int k0) {
