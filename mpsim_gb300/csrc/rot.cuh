@@ -91,6 +91,11 @@ __device__ __forceinline__ void apply_rot(const Rot& r, cf& x, cf& q) {
 // than a few ulps of s^2.  A pair whose squared cosine is not above thr gets the
 // identity; in a careful visit (one with tiny columns), pairs whose squares could
 // leave FP32's range take the scaled form above.
+// Within a visit the norms are carried along, and those of columns that cancel against
+// each other (equal columns) end as noise that need not agree with gamma.  Whatever
+// they are, the rotation has to be a rotation: a pair whose p^2 + 4 |gamma|^2 is too
+// small for u, or whose gamma is too large for its norms (the scaled form would
+// square their ratio), stays as it is until its products are formed afresh.
 // Squared norms above this (theta's is in [1, 4)) keep every product that a
 // rotation is decided on within FP32's normal range.
 constexpr float kTinyNorm2 = 1e-9f;
@@ -114,9 +119,10 @@ __device__ __forceinline__ PairRot pair_rotation(float a, float b, cf gam, float
     const float g2 = cabs2(gam), ab = a * b, p = b - a;
     const bool small = careful && (g2 < 1e-30f || ab < 1e-30f);
     PairRot o;
-    o.rot = !small && g2 > thr * ab;
+    const float x = fmaf(p, p, 4.f * g2);
+    o.rot = !small && g2 > thr * ab && x >= 1e-37f;
     // (a pair of zero columns stays finite)
-    const float u = newton_rsqrt(fmaxf(fmaf(p, p, 4.f * g2), 1e-37f));
+    const float u = newton_rsqrt(fmaxf(x, 1e-37f));
     const float c2 = fmaf(0.5f * fabsf(p), u, 0.5f);
     const float ic = newton_rsqrt(c2);
     const float k = o.rot ? u * ic : 0.f;                // s = |gamma| k
@@ -130,7 +136,7 @@ __device__ __forceinline__ PairRot pair_rotation(float a, float b, cf gam, float
     o.c = o.rot ? c2 * ic : 1.f;
     o.ic = o.rot ? ic : 1.f;
     if (careful) {
-        if (small && pair_cos2(gam, g2, a, b) > thr) {
+        if (small && fabsf(gam.x) + fabsf(gam.y) <= a + b && pair_cos2(gam, g2, a, b) > thr) {
             const Rot r = make_rot(a, b, gam);
             o.tp = r.tp;
             o.sr = r.sigma.x;

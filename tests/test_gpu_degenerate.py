@@ -1,0 +1,62 @@
+"""Truncated SVDs of degenerate thetas: equal, zero and repeated columns, exact ties,
+spectra of thirty decades.  Columns cancel to rounding noise and to norms whose squares
+are no normal floats; the factors stay finite and the isometric one an isometry.
+Checked like test_gpu_svd_kernel.py's jobs (same tolerances) against complex128 LAPACK.
+"""
+import numpy as np
+import pytest
+
+from mpsim_gb300 import _native
+from test_gpu_svd_kernel import check_job, run_batch
+
+pytestmark = pytest.mark.gpu
+
+
+def _theta(kind, m, n, rng):
+    x = rng.normal(size=(m, n)) + 1j * rng.normal(size=(m, n))
+    r = min(m, n)
+    if kind == "constant":
+        return np.ones((m, n), complex)
+    if kind == "zero columns":
+        x[:, ::3] = 0
+        x[1::4] = 0
+    elif kind == "repeated columns":
+        x[:, 1::2] = x[:, 0:2 * (n // 2):2]
+    elif kind == "permutation":
+        x = np.zeros((m, n), complex)
+        x[np.arange(r), rng.permutation(n)[:r]] = 1
+    elif kind == "thirty decades":
+        u, _, vh = np.linalg.svd(x, full_matrices=False)
+        x = (u * 10.0 ** -np.linspace(0, 30, r)) @ vh
+    return x
+
+
+KINDS = ["constant", "zero columns", "repeated columns", "permutation", "thirty decades"]
+
+
+def _spec(kind, chil, chir, k, lc):
+    """The job whose merged theta (identity gate) is this matrix."""
+    m, n = 2 * chil, 2 * chir
+    th = _theta(kind, m, n, np.random.default_rng(m + 1000 * n))
+    if m >= n:
+        a, b = th.reshape(chil, 2, n), np.eye(n).reshape(n, 2, chir)
+    else:
+        a, b = np.eye(m).reshape(chil, 2, m), th.reshape(m, 2, chir)
+    return a.astype(np.complex64), b.astype(np.complex64), np.eye(4, dtype=np.complex64), k, lc
+
+
+def _check(lib, cuda, specs, precision=_native.PRECISION_PLAIN):
+    p = _native.SvdParams()
+    p.precision = precision
+    rc, res, _ = run_batch(lib, cuda, specs, params=p)
+    assert rc == 0, _native.last_error()
+    for spec, out in zip(specs, res):
+        check_job(spec, out, 2)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("chil,chir,lc", [(8, 20, True), (33, 40, True), (40, 70, True), (64, 100, True),
+                                          (70, 40, False), (100, 64, False), (60, 130, False)])
+def test_rotations_accumulated(built_lib, cuda, kind, chil, chir, lc):
+    """Jobs that accumulate V: every rotation of noise has to be one."""
+    _check(built_lib, cuda, [_spec(kind, chil, chir, 2 * min(chil, chir), lc)])
