@@ -60,3 +60,20 @@ def _check(lib, cuda, specs, precision=_native.PRECISION_PLAIN):
 def test_rotations_accumulated(built_lib, cuda, kind, chil, chir, lc):
     """Jobs that accumulate V: every rotation of noise has to be one."""
     _check(built_lib, cuda, [_spec(kind, chil, chir, 2 * min(chil, chir), lc)])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("chil,chir,lc", [(8, 8, True), (33, 40, False), (40, 70, False), (64, 64, True),
+                                          (64, 64, False), (100, 64, True), (64, 100, False),
+                                          (128, 128, False), (300, 40, True)])
+def test_left_factor_read_off_the_columns(built_lib, cuda, kind, chil, chir, lc):
+    """Jobs without V: columns too short to be made orthogonal are completed, not divided
+    by their norms; all singular vectors kept, and half of them."""
+    k = 2 * min(chil, chir)
+    _check(built_lib, cuda, [_spec(kind, chil, chir, k, lc), _spec(kind, chil, chir, k // 2, lc)])
+
+
+@pytest.mark.parametrize("kind", ["constant", "zero columns", "permutation", "thirty decades"])
+@pytest.mark.parametrize("chil,chir", [(64, 64), (100, 64), (128, 128)])
+def test_mixed(built_lib, cuda, kind, chil, chir):
+    _check(built_lib, cuda, [_spec(kind, chil, chir, 2 * chir, True)], _native.PRECISION_MIXED)
