@@ -43,8 +43,8 @@
 // rotations of each visit in V.
 //
 // Afterwards sigma_c = |X_c|, sorted descending (ties by column index); the
-// first k are kept.  Where the isometric factor would divide by an exact-zero
-// singular value, an orthonormal completion (classical Gram-Schmidt, twice) is
+// first k are kept.  Where the isometric factor would divide by a zero singular
+// value (one at or below kZeroSigma), an orthonormal completion (classical Gram-Schmidt, twice) is
 // written instead -- LAPACK also returns orthonormal singular vectors for zero
 // singular values, and which ones it returns does not change any later
 // singular value of the state.

@@ -6,21 +6,27 @@
 
 namespace mps {
 
+// Columns whose squared norm is below this (theta's is in [1, 4)) count as zero:
+// nothing rotates them, and the isometric factor is completed where they stand
+// (kZeroSigma).  A pair that rotates has |gamma| of 1e-7 sqrt(a b) or more, and
+// make_rot's sigma / conj(gamma), up to 1 / |gamma|, has to stay a float: 1e-31 at
+// least.  Columns of an exactly dependent set shrink by 1e-7 a sweep, and were
+// followed down to 1e-18 and below, where squares underflow and a cosine comes out
+// too large for ever: sweeps up to the cap, or NaN.
+constexpr float kZeroNorm2 = 1e-30f;
+
 // Squared cosine of the angle between two columns, |gamma|^2 / (a b).  A pair
 // rotates when it exceeds tol^2, and the per-job maximum of the same value
 // decides convergence, so a sweep that rotates nothing always ends the job.
-// Zero columns give 0; when g2 = |gamma|^2 or a norm is below the smallest
-// normal float, the cosine is formed from |gamma| and the square roots of the
-// norms with IEEE operations instead.
+// Zero columns give 0; when g2 = |gamma|^2 is below the smallest normal float, the
+// cosine is formed from |gamma| and the square roots of the norms with IEEE
+// operations instead.
 __device__ __forceinline__ float pair_cos2(cf gam, float g2, float a, float b) {
     const float kMinNormal = 1.17549435e-38f;
-    if (g2 >= kMinNormal && a >= kMinNormal && b >= kMinNormal)
-        return __fdividef(__fdividef(g2, a), b);
+    if (!(a >= kZeroNorm2 && b >= kZeroNorm2)) return 0.f;
+    if (g2 >= kMinNormal) return __fdividef(__fdividef(g2, a), b);
     // |gamma|^2 underflows once the columns are below ~1e-10 in norm (graded
     // columns, as the L factor has from the start): take |gamma| itself.
-    // Pairs with a + b below 1e-36 leave no room for the rotation's
-    // 1/(a+b) and count as orthogonal.
-    if (!(a > 0.f && b > 0.f) || !(a + b >= 1e-36f)) return 0.f;
     const float r = (hypotf(gam.x, gam.y) / sqrtf(a)) / sqrtf(b);
     return r * r;
 }
@@ -39,7 +45,7 @@ struct Rot {
 };
 
 // Rotation parameters for gamma != 0 from quantities scaled by u = 1/(a+b)
-// (gamma u is squared, not gamma: no overflow or underflow for a + b >= 1e-36):
+// (gamma u is squared, not gamma: no overflow or underflow for a + b >= kZeroNorm2):
 // t = sign(b-a) 2|gamma| / (|b-a| + sqrt((b-a)^2 + 4|gamma|^2)),
 // c = 1/sqrt(1+t^2) (approximate reciprocal square root refined by one
 // Newton step), s = c t.  |sigma|^2 and tp come from the same c^2 t^2, so

@@ -439,7 +439,7 @@ __device__ __forceinline__ bool visit(const TwoQGeom& g, int j, int I, int J, bo
             const cf gam = G[gidx(p, q)];
             const double g2 = (double)gam.x * gam.x + (double)gam.y * gam.y;
             const double ab = (double)a * (double)b;
-            if (a > 0.f && b > 0.f && g2 > tol2d * ab) {
+            if (a >= kZeroNorm2 && b >= kZeroNorm2 && g2 > tol2d * ab) {
                 any = 1;
                 cmax = fmaxf(cmax, (float)g2 / (float)ab);
             }

@@ -131,11 +131,10 @@ __host__ __device__ __forceinline__ float default_tol2(int rows) {
 
 // Singular values at or below this (relative to max(s_0, 1); theta's norm is in
 // [1, 2)) are treated as zeros: the isometric factor gets an orthonormal completion
-// there.  The squares of such columns' norms (1e-36) and the products of two of them
-// leave FP32's normal range, so the sweeps take them for orthogonal as they are
-// (pair_cos2); divided by their norms they need not be: of 128 equal columns 113 ended
-// between 1e-21 and 1e-20, all parallel.
-constexpr float kZeroSigma = 1e-18f;
+// there.  A little above the norm of columns that the sweeps leave as they are
+// (kZeroNorm2 in rot.cuh); divided by their norms those need not be orthogonal: of
+// 128 equal columns 113 ended between 1e-21 and 1e-20, all parallel.
+constexpr float kZeroSigma = 2e-15f;
 
 // Replaces X by its L factor (X = L Q) for the jobs whose left factor comes
 // from the final columns (lq.cu); the sweeps then need fewer passes.

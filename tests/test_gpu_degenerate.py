@@ -22,6 +22,8 @@ def _theta(kind, m, n, rng):
         x[1::4] = 0
     elif kind == "repeated columns":
         x[:, 1::2] = x[:, 0:2 * (n // 2):2]
+    elif kind == "repeated rows":
+        x[1::2] = x[0:2 * (m // 2):2]
     elif kind == "permutation":
         x = np.zeros((m, n), complex)
         x[np.arange(r), rng.permutation(n)[:r]] = 1
@@ -31,7 +33,8 @@ def _theta(kind, m, n, rng):
     return x
 
 
-KINDS = ["constant", "zero columns", "repeated columns", "permutation", "thirty decades"]
+KINDS = ["constant", "zero columns", "repeated columns", "repeated rows", "permutation",
+         "thirty decades"]
 
 
 def _spec(kind, chil, chir, k, lc):
@@ -71,6 +74,17 @@ def test_left_factor_read_off_the_columns(built_lib, cuda, kind, chil, chir, lc)
     by their norms; all singular vectors kept, and half of them."""
     k = 2 * min(chil, chir)
     _check(built_lib, cuda, [_spec(kind, chil, chir, k, lc), _spec(kind, chil, chir, k // 2, lc)])
+
+
+@pytest.mark.parametrize("kind,chil,chir,lc", [
+    ("constant", 384, 384, True), ("constant", 384, 384, False), ("repeated rows", 384, 384, True),
+    ("repeated columns", 400, 400, False), ("repeated rows", 400, 400, True),
+    ("constant", 450, 450, False), ("constant", 600, 60, True), ("repeated rows", 600, 60, True)])
+def test_exactly_dependent_columns_end(built_lib, cuda, kind, chil, chir, lc):
+    """Columns of an exactly dependent set shrink with every sweep; they are followed no
+    further than they can be made orthogonal, within the sweep cap (768 columns: the
+    factorised start's most; 800 and 900: without it; 1200 rows: column by column)."""
+    _check(built_lib, cuda, [_spec(kind, chil, chir, min(chil, chir), lc)])
 
 
 @pytest.mark.parametrize("kind", ["constant", "zero columns", "permutation", "thirty decades"])
