@@ -49,8 +49,11 @@ __device__ __forceinline__ void copy8_async(uint32_t dst, const void* src, uint3
 // CONJ: the second factor is conjugated (conjA != conjB); a conjugated first
 // factor is the conjugate of the product with the second one's conjugation
 // flipped.  GATHER: row i of A (and the row given to put) is rows[i], negative:
-// none.  All threads of the block call it.
-template <int TM, int TN, int KS>
+// none.  PART > 0: the sum over K is taken in parts of PART chunks, so that its
+// rounding error stays that of short sums where every term has the same sign (two
+// columns of equal entries: a single sum of 512 terms is off by 1.5e-5).  All
+// threads of the block call it.
+template <int TM, int TN, int KS, int PART = 0>
 struct GemmTile {
     static constexpr int KC = KS > 1 ? 16 : 8;                // K of a chunk
     static constexpr int ST = 4;                              // chunks in shared memory
@@ -123,6 +126,13 @@ struct GemmTile {
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = cmake(0.f, 0.f);
+        cf sum[PART > 0 ? 4 : 1][4];
+        if constexpr (PART > 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sum[i][j] = cmake(0.f, 0.f);
+        }
 #pragma unroll
         for (int c = 0; c < ST - 1; ++c) fetch(c);
         for (int c = 0; c < chunks; ++c) {
@@ -144,6 +154,23 @@ struct GemmTile {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) cfma_op<CONJ>(acc[i][j], av[i], bv[j]);
             }
+            if constexpr (PART > 0) {
+                if (c % PART == PART - 1 || c == chunks - 1) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            sum[i][j] = cadd(sum[i][j], acc[i][j]);
+                            acc[i][j] = cmake(0.f, 0.f);
+                        }
+                }
+            }
+        }
+        if constexpr (PART > 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = sum[i][j];
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();

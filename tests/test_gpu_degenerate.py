@@ -91,3 +91,20 @@ def test_exactly_dependent_columns_end(built_lib, cuda, kind, chil, chir, lc):
 @pytest.mark.parametrize("chil,chir", [(64, 64), (100, 64), (128, 128)])
 def test_mixed(built_lib, cuda, kind, chil, chir):
     _check(built_lib, cuda, [_spec(kind, chil, chir, 2 * chir, True)], _native.PRECISION_MIXED)
+
+
+@pytest.mark.parametrize("chil,chir,lc", [(64, 64, False), (288, 288, True), (288, 288, False),
+                                          (150, 290, False), (512, 200, True), (600, 100, True)])
+def test_constant_theta_keeps_its_accuracy(built_lib, cuda, chil, chir, lc):
+    """Every product of a constant theta's factors sums equal terms, whose roundings all go
+    one way.  In parts of 32 terms (two FMAs each) and their sums a product of K terms is
+    off by (64 + K / 32) 2^-25 at most, 3e-6 here; twice that for the isometry and for the
+    two factors' product beside what random thetas show (a single sum of K: 2 K 2^-25)."""
+    spec = _spec("constant", chil, chir, 8, lc)
+    rc, res, _ = run_batch(built_lib, cuda, [spec])
+    assert rc == 0, _native.last_error()
+    left = res[0]["a"].reshape(2 * chil, 8).astype(np.complex128)
+    right = res[0]["b"].reshape(8, 2 * chir).astype(np.complex128)
+    gram = left.conj().T @ left if lc else right @ right.conj().T
+    assert np.max(np.abs(gram - np.eye(8))) <= 6e-6
+    assert np.linalg.norm(left @ right - 1) <= 6e-6 * np.sqrt(left.shape[0] * right.shape[1])
