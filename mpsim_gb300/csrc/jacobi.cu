@@ -983,14 +983,64 @@ int launch_post(const mps_2q_job* jobs, int njobs, int max_m, int max_n, int kma
     return MPS_OK;
 }
 
-// Orthonormal completion of the isometric factor where sigma is an exact
-// zero (where the isometric site divides by S).  Vectors u_i (i < k): left-canonical -> columns of a_out
-// (R = m, element stride k); right-canonical -> rows of b_out (R = n, element
-// stride 1).  The columns
-// needing completion are a suffix of the kept set (sigma sorted).
-constexpr int COMP_T = 256;
+// Orthonormal completion of the isometric factor where sigma is zero (where the
+// isometric site divides by S).  Vectors u_i (i < k): left-canonical -> columns of
+// a_out (R = m, element stride k); right-canonical -> rows of b_out (R = n, element
+// stride 1).  The columns needing completion are a suffix of the kept set (sigma
+// sorted), and each is a unit vector made orthogonal, twice, to those before it:
+// one after another, bound by the latency of reading them.  Both contractions of a
+// pass read along the contiguous side of the site, over a warp's lanes or over the
+// threads: 256 of 512 columns, 8 jobs, 44-51 ms a call before (one thread an element,
+// loads one by one and strided in the left-canonical form), 10-15 now.
+constexpr int COMP_T = 1024;
 
-__global__ void __launch_bounds__(COMP_T)
+// out[o] = sum_i M[o * ld + i] x[i] over the contiguous index, a warp an output.
+template <bool CONJ>
+__device__ __forceinline__ void contract_rows(const cf* M, size_t ld, int rows, int cols, const cf* x,
+                                              cf* out) {
+    const int lane = threadIdx.x & 31;
+    for (int o = threadIdx.x >> 5; o < rows; o += COMP_T / 32) {
+        cf acc = cmake(0.f, 0.f);
+#pragma unroll 8
+        for (int i = lane; i < cols; i += 32) {
+            const cf v = M[o * ld + i];
+            if (CONJ) cfma_conj(acc, v, x[i]);
+            else cfma(acc, v, x[i]);
+        }
+        acc.x = warp_sum(acc.x);
+        acc.y = warp_sum(acc.y);
+        if (lane == 0) out[o] = acc;
+    }
+}
+
+// out[i] = sum_o M[o * ld + i] y[o] over the strided index: a thread an output and a share
+// of the rows, the shares' sums through part (COMP_T elements).
+template <bool CONJ>
+__device__ __forceinline__ void contract_columns(const cf* M, size_t ld, int rows, int cols,
+                                                 const cf* y, cf* part, cf* out) {
+    for (int c0 = 0; c0 < cols; c0 += COMP_T) {
+        const int width = min(cols - c0, COMP_T), shares = COMP_T / width;
+        const int share = threadIdx.x / width, i = c0 + threadIdx.x - share * width;
+        cf acc = cmake(0.f, 0.f);
+        if (share < shares) {
+#pragma unroll 8
+            for (int o = share; o < rows; o += shares) {
+                const cf v = M[o * ld + i];
+                if (CONJ) cfma_conj(acc, v, y[o]);
+                else cfma(acc, v, y[o]);
+            }
+            part[threadIdx.x] = acc;
+        }
+        __syncthreads();
+        if (threadIdx.x < width) {
+            for (int q = 1; q < shares; ++q) acc = cadd(acc, part[q * width + threadIdx.x]);
+            out[i] = acc;
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(COMP_T, 1)
 complete_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
     extern __shared__ float2 sm3[];
     const int j = blockIdx.x;
@@ -998,59 +1048,52 @@ complete_kernel(const mps_2q_job* __restrict__ jobs, TwoQGeom g) {
     if (need == 0) return;
     const mps_2q_job job = jobs[j];
     const int m = job.chi_l * g.d, n = job.chi_r * g.d;
-    const bool tall = job.keep_left_canonical != 0;
+    const bool left = job.keep_left_canonical != 0;
     const int k = job.k;
-    const int R = tall ? m : n;
-    cf* base = reinterpret_cast<cf*>(tall ? job.a_out : job.b_out);
-    const size_t es = tall ? (size_t)k : 1;     // element stride
-    const size_t vs = tall ? 1 : (size_t)n;     // vector stride
+    const int R = left ? m : n;
+    cf* base = reinterpret_cast<cf*>(left ? job.a_out : job.b_out);
+    const size_t es = left ? (size_t)k : 1;     // element stride
+    const size_t vs = left ? 1 : (size_t)n;     // vector stride
     cf* v = sm3;                                // [R]
-    cf* h = sm3 + R;                            // [k]
+    cf* w = v + R;                              // [R]: the part of v in the span
+    cf* h = w + R;                              // [k]
+    cf* part = h + k;                           // [COMP_T]
     __shared__ float s_nrm[COMP_T / 32];
-    __shared__ int s_ok;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int cand = 0;
     for (int i = k - need; i < k; ++i) {
         for (;;) {
             if (cand >= R) return;              // unreachable: see the threshold below
             for (int e = tid; e < R; e += COMP_T) v[e] = cmake(e == cand ? 1.f : 0.f, 0.f);
-            __syncthreads();
-            for (int pass = 0; pass < 2; ++pass) {
-                for (int t = warp; t < i; t += COMP_T / 32) {
-                    cf acc = cmake(0.f, 0.f);
-                    for (int e = lane; e < R; e += 32)
-                        cfma_conj(acc, base[t * vs + e * es], v[e]);
-                    acc.x = warp_sum(acc.x);
-                    acc.y = warp_sum(acc.y);
-                    if (lane == 0) h[t] = acc;
-                }
-                __syncthreads();
-                for (int e = tid; e < R; e += COMP_T) {
-                    cf acc = v[e];
-                    for (int t = 0; t < i; ++t) acc = csub(acc, cmul(h[t], base[t * vs + e * es]));
-                    v[e] = acc;
-                }
-                __syncthreads();
-            }
-            float s = 0.f;
-            for (int e = tid; e < R; e += COMP_T) s += cabs2(v[e]);
-            s = warp_sum(s);
-            if (lane == 0) s_nrm[warp] = s;
-            __syncthreads();
-            if (tid == 0) {
-                float tot = 0.f;
-                for (int w = 0; w < COMP_T / 32; ++w) tot += s_nrm[w];
-                s_nrm[0] = tot;
-                // the residuals of all R candidates sum to R - i >= 1, so
-                // some candidate always clears 0.5 / R
-                s_ok = tot > 0.5f / (float)R;
-            }
-            __syncthreads();
-            const float nv = s_nrm[0];
-            const int ok = s_ok;
             ++cand;
             __syncthreads();
-            if (ok) {
+            float nv = 0.f;
+            for (int pass = 0; pass < 2; ++pass) {
+                // h = U^H v, w = U h
+                if (left) {
+                    contract_columns<true>(base, es, R, i, v, part, h);
+                    contract_rows<false>(base, es, R, i, h, w);
+                } else {
+                    contract_rows<true>(base, vs, i, R, v, h);
+                    __syncthreads();
+                    contract_columns<false>(base, vs, i, R, h, part, w);
+                }
+                __syncthreads();
+                float s = 0.f;
+                for (int e = tid; e < R; e += COMP_T) {
+                    const cf x = csub(v[e], w[e]);
+                    v[e] = x;
+                    s += cabs2(x);
+                }
+                s = warp_sum(s);
+                if (lane == 0) s_nrm[warp] = s;
+                __syncthreads();
+                nv = warp_sum(s_nrm[lane]);
+                __syncthreads();
+            }
+            // the residuals of all R candidates sum to R - i >= 1, so some
+            // candidate always clears 0.5 / R
+            if (nv > 0.5f / (float)R) {
                 const float inv = rsqrtf(nv);
                 for (int e = tid; e < R; e += COMP_T) base[i * vs + e * es] = cscale(v[e], inv);
                 __syncthreads();
@@ -1649,7 +1692,7 @@ extern "C" int mps_apply_2q_batch(void* stream, const mps_2q_job* jobs, int njob
         dim3 gb((max_n + 255) / 256, kmax, njobs);
         regauge_b_kernel<<<gb, 256, 0, s>>>(jobs, g);
         MPS_LAUNCH_CHECK("regauge_b_kernel");
-        const size_t comp_smem = (size_t)(max(max_m, max_n) + kmax) * sizeof(cf);
+        const size_t comp_smem = (size_t)(2 * max(max_m, max_n) + kmax + COMP_T) * sizeof(cf);
         if (comp_smem > 48 * 1024) {
             MPS_CUDA_CHECK(cudaFuncSetAttribute(complete_kernel,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1862,7 +1905,7 @@ extern "C" int mps_apply_2q_batch_noalloc(void* stream, const mps_2q_job* jobs, 
         dim3 gb((max_n + 255) / 256, kmax, njobs);
         regauge_b_kernel<<<gb, 256, 0, s>>>(jobs, g);
         MPS_LAUNCH_CHECK("regauge_b_kernel");
-        const size_t comp_smem = (size_t)(max(max_m, max_n) + kmax) * sizeof(cf);
+        const size_t comp_smem = (size_t)(2 * max(max_m, max_n) + kmax + COMP_T) * sizeof(cf);
         if (comp_smem > 48 * 1024) {
             MPS_CUDA_CHECK(cudaFuncSetAttribute(complete_kernel,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
